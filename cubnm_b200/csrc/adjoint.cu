@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(1024) k_adj_backward(const AdjArgs A) {
                     const float II = (float)m.w_I__I_0 + J_N * SE - (float)m.w_II * SI;
                     const float xE = (float)m.a_E * IE - (float)m.b_E;
                     const float xI = (float)m.a_I * II - (float)m.b_I;
-                    const float rE = rate_of<float>(xE, m.d_E);
-                    const float rI = rate_of<float>(xI, m.d_I);
+                    const float rE = rate_of(xE, (float)m.d_E);
+                    const float rI = rate_of(xI, (float)m.d_I);
                     const float uE = SE + (n0 * sig * sqdt + (float)m.dt_gamma_E * ((1.0f - SE) * rE) -
                                            (float)m.dt_itau_E * SE);
                     const float uI = SI + (n1 * sig * sqdt + (float)m.dt_gamma_I * rI - (float)m.dt_itau_I * SI);

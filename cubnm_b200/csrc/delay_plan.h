@@ -1,0 +1,199 @@
+// Host side of the delay kernel (integrate_delay.cuh): its tiles and entry lists.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <map>
+#include <utility>
+#include <vector>
+
+namespace cbnm {
+
+constexpr int DELAY_BLOCK = 32;          // integration steps per block of the kernel
+constexpr int DELAY_SMEM_SM = 227 * 1024;   // shared memory of an SM that CTAs can use, and 1 KB of it per CTA is the system's
+
+struct DelayPlan {
+    int window = 0, tiles = 0, tile_src = 0, bufs = 1, threads = 0, blob_max = 0, buf_bytes = 0, buf_at = 0, noise_steps = 0;
+    int smem = 0, n_pairs = 0, near_k = 1, far_max = 0;
+    std::vector<int> pair, blob_at, near, near_cnt, near_min;
+    std::vector<unsigned char> blob;
+    std::vector<double> near_w;
+};
+
+// The pairs (SC, delay table) that the simulations use.
+inline std::vector<std::pair<int, int>> delay_pairs(DelayPlan &p, int n_sims, const int *sc_of,
+                                                    const std::vector<int> &table_of) {
+    std::map<std::pair<int, int>, int> id;
+    std::vector<std::pair<int, int>> pairs;
+    p.pair.resize(n_sims);
+    for (int s = 0; s < n_sims; ++s) {
+        const auto key = std::make_pair(sc_of[s], table_of[s]);
+        const auto it = id.emplace(key, (int)pairs.size());
+        if (it.second) pairs.push_back(key);
+        p.pair[s] = it.first->second;
+    }
+    p.n_pairs = (int)pairs.size();
+    return pairs;
+}
+
+// A tile's entry lists, 16-byte aligned: this header, unsigned end[n] (low half: pairs of
+// far entries up to and with the target's, high half: near entries), then at the byte
+// offsets given: far offsets into the tile's windows of x(t0 - d) (16 bits each, a
+// target's padded to a pair by repeating one with weight 0), their weights, near codes
+// (offset * 32 + delay) and their weights.
+struct TileHead { int off_at, w_at, near_at, near_w_at; };
+
+// Lists of all pairs for tiles of p.tile_src sources; R = float or double.  False
+// where a list exceeds its index width or all lists max_bytes.
+template <class R>
+inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector<int> &delay,
+                        const std::vector<std::pair<int, int>> &pairs, size_t max_bytes) {
+    const size_t nn = (size_t)n * n;
+    const int W = p.window;
+    p.tiles = (n + p.tile_src - 1) / p.tile_src;
+    p.blob.clear();
+    p.blob_at.clear();
+    p.blob_max = 0;
+    std::vector<unsigned> end(n);
+    std::vector<uint16_t> off;
+    std::vector<int> noff;
+    std::vector<R> w, nw;
+    auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    for (const auto &pr : pairs) {
+        const double *S = sc + (size_t)pr.first * nn;
+        const int *d = delay.data() + (size_t)pr.second * nn;
+        for (int t = 0; t < p.tiles; ++t) {
+            const int s0 = t * p.tile_src, s1 = std::min(n, s0 + p.tile_src);
+            off.clear(); w.clear(); noff.clear(); nw.clear();
+            for (int j = 0; j < n; ++j) {
+                for (int k = s0; k < s1; ++k) {
+                    const double v = S[(size_t)k * n + j];
+                    if (v == 0.0) continue;
+                    const int dk = d[(size_t)k * n + j], o = (k - s0) * W + (W - dk);
+                    if (dk >= DELAY_BLOCK) {
+                        off.push_back((uint16_t)o);
+                        w.push_back((R)v);
+                    } else {
+                        noff.push_back(o * 32 + dk);
+                        nw.push_back((R)v);
+                    }
+                }
+                if (off.size() % 2) {
+                    off.push_back(off.back());
+                    w.push_back(R(0));
+                }
+                if (off.size() / 2 > 0xffff || noff.size() > 0xffff) return false;
+                end[j] = (unsigned)(off.size() / 2) | ((unsigned)noff.size() << 16);
+            }
+            TileHead h;
+            h.off_at = (int)up16(sizeof(h) + sizeof(unsigned) * n);
+            h.w_at = (int)up16(h.off_at + sizeof(uint16_t) * off.size());
+            h.near_at = (int)up16(h.w_at + sizeof(R) * w.size());
+            h.near_w_at = (int)up16(h.near_at + sizeof(int) * noff.size());
+            const size_t bytes = up16(h.near_w_at + sizeof(R) * nw.size()), at = p.blob.size();
+            p.blob_at.push_back((int)(at / 16));
+            p.blob.resize(at + bytes);
+            unsigned char *b = p.blob.data() + at;
+            std::memcpy(b, &h, sizeof(h));
+            std::memcpy(b + sizeof(h), end.data(), sizeof(unsigned) * n);
+            if (!off.empty()) {
+                std::memcpy(b + h.off_at, off.data(), sizeof(uint16_t) * off.size());
+                std::memcpy(b + h.w_at, w.data(), sizeof(R) * w.size());
+            }
+            if (!noff.empty()) {
+                std::memcpy(b + h.near_at, noff.data(), sizeof(int) * noff.size());
+                std::memcpy(b + h.near_w_at, nw.data(), sizeof(R) * nw.size());
+            }
+            p.blob_max = std::max(p.blob_max, (int)bytes);
+            if (p.blob.size() > max_bytes) return false;
+        }
+        p.blob_at.push_back((int)(p.blob.size() / 16));
+    }
+    return true;
+}
+
+// Chooses the tile and launch shape and builds the lists.  sc [n_scs][n*n] (row =
+// source), delay [n_tables][n*n] steps (>= 1).  As many CTAs per SM as the batch can
+// fill while a tile still holds about three entries per target (each target and tile costs
+// a read and a write of its sums and half an entry of padding); alone on its SM a CTA
+// keeps two tile buffers.  Returns false where the kernel does
+// not apply: tiles of under 4 sources, most pairs near, or lists beyond max_bytes.
+template <class R>
+inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int sms, const double *sc, const int *sc_of,
+                             const std::vector<int> &delay, const std::vector<int> &table_of, int max_delay,
+                             size_t max_bytes) {
+    p.window = (std::max(max_delay, DELAY_BLOCK) + DELAY_BLOCK - 1) / DELAY_BLOCK * DELAY_BLOCK;
+    const auto pairs = delay_pairs(p, n_sims, sc_of, table_of);
+    const size_t nn = (size_t)n * n;
+    // near lists for the steps within a block, by rank q
+    p.near_cnt.assign(p.n_pairs, 0);
+    p.near_min.assign(p.n_pairs, DELAY_BLOCK);
+    struct Near { int pair, node, rank, off; double w; };
+    std::vector<Near> near;
+    size_t nnz = 0;   // of the fullest pair
+    if ((size_t)p.n_pairs * nn > max_bytes) return false;
+    for (int q = 0; q < p.n_pairs; ++q) {
+        const double *S = sc + (size_t)pairs[q].first * nn;
+        const int *d = delay.data() + (size_t)pairs[q].second * nn;
+        size_t all = 0;
+        for (int j = 0; j < n; ++j) {
+            int rank = 0, far = 0;
+            for (int k = 0; k < n; ++k) {
+                const double v = S[(size_t)k * n + j];
+                if (v == 0.0) continue;
+                const int dk = d[(size_t)k * n + j];
+                if (dk >= DELAY_BLOCK) { ++far; continue; }
+                near.push_back({q, j, rank++, k * DELAY_BLOCK + dk, v});
+                p.near_min[q] = std::min(p.near_min[q], dk);
+            }
+            p.near_cnt[q] = std::max(p.near_cnt[q], rank);
+            p.far_max = std::max(p.far_max, far);
+            all += far + rank;
+        }
+        nnz = std::max(nnz, all);
+    }
+    for (int c : p.near_cnt) p.near_k = std::max(p.near_k, c);
+    if (p.near_k > std::max(8, p.far_max / 4) || (size_t)p.n_pairs * p.near_k * n * 16 > max_bytes) return false;
+    p.near.assign((size_t)p.n_pairs * p.near_k * n, 0);
+    p.near_w.assign(p.near.size(), 0.0);
+    for (const Near &e : near) {
+        const size_t at = ((size_t)e.pair * p.near_k + e.rank) * n + e.node;
+        p.near[at] = e.off;
+        p.near_w[at] = e.w;
+    }
+    // tile and launch shape
+    const int least = (n + 31) / 32 * 32;
+    const bool f64 = sizeof(R) == 8;
+    const int rows = (int)(sizeof(R) * n * (DELAY_BLOCK + 1) + 15) & ~15;
+    p.buf_at = rows;
+    const double nnz_node = (double)nnz / n;
+    const double per_src = (double)p.window * sizeof(R) + (nnz_node + n * 0.3) * (2 + sizeof(R));   // window and entries
+    const int thr_sm = f64 ? 512 : 1024;   // by registers, see min_ctas
+    for (int c = std::min({8, (n_sims + sms - 1) / sms, std::max(1, thr_sm / least)}); c >= 1; --c) {
+        const double space = DELAY_SMEM_SM / c - 1024 - p.buf_at - 4.0 * n - 256;
+        auto fit = [&](int bufs) { return std::min<int>({n, 65535 / p.window, (int)((space - (bufs - 1) * 4.0 * n) / bufs / per_src)}); };
+        p.bufs = 1;
+        p.tile_src = fit(1);
+        if (p.tile_src < n && c == 1 && nnz_node * fit(2) / n >= 12.0) {   // alone on its SM: load during the gather
+            p.bufs = 2;
+            p.tile_src = fit(2);
+        }
+        if (c > 1 && p.tile_src < n && nnz_node * p.tile_src / n < 3.0) continue;
+        if (p.tile_src < std::min(n, 4)) continue;
+        const int most = c == 1 ? (f64 ? 512 : n <= 256 ? 512 : 1024) : std::min(f64 ? 256 : 512, thr_sm / c / 32 * 32);
+        p.threads = std::max(least, most);
+        for (int shrink = 0; shrink < 8 && p.tile_src >= 1; ++shrink) {
+            if (!delay_blobs<R>(p, n, sc, delay, pairs, max_bytes)) return false;
+            p.buf_bytes = ((p.blob_max + p.tile_src * p.window * (int)sizeof(R)) + 15) & ~15;
+            p.smem = p.buf_at + p.bufs * p.buf_bytes;
+            if (p.smem <= DELAY_SMEM_SM / c - 1024) {
+                p.noise_steps = std::min(DELAY_BLOCK, p.bufs * p.buf_bytes / (int)(sizeof(R) * n * n_noise));
+                return p.noise_steps > 0;
+            }
+            p.tile_src = (int)(p.tile_src * 0.93);
+        }
+    }
+    return false;
+}
+
+}  // namespace cbnm

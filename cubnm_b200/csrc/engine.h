@@ -40,23 +40,39 @@ struct BWFast {
 
 // Model constants, computed on the host exactly as the reference's
 // init_constants(dt) does (src/ext/models/<model>.cpp).
-struct RWWK {
-    double dt, sqrt_dt, a_E, b_E, d_E, a_I, b_I, d_I, w_II, w_E__I_0, w_I__I_0, b_a_ratio_E;
-    double dt_itau_E, dt_gamma_E, dt_itau_I, dt_gamma_I;
+// The constants in type T (double, or their float rounding).
+template <class T>
+struct RWWKt {
+    T dt, sqrt_dt, a_E, b_E, d_E, a_I, b_I, d_I, w_II, w_E__I_0, w_I__I_0, b_a_ratio_E;
+    T dt_itau_E, dt_gamma_E, dt_itau_I, dt_gamma_I;
     // analytical-FIC constants (rww.cpp:42-53)
-    double I_0, w_E, w_I, I_ext, tau_I_s, gamma_I_s, I_E_ss, S_E_ss;
+    T I_0, w_E, w_I, I_ext, tau_I_s, gamma_I_s, I_E_ss, S_E_ss;
 };
-struct WCK { double dt, sqrt_dt, itau_E, itau_I, a_E, a_I, mu_E, mu_I; };
-struct JRK { double dt, sqrt_dt, A, B, a, b, v0, nu_max, r, mu, cmin, cmax, midpoint, a_sq, b_sq; };
-struct KurK { double dt, sqrt_dt, twopi; };
-struct RWWExK { double dt, sqrt_dt, J_N, a, b, d, dt_itau, dt_gamma; };
-union ModelK {
-    RWWK rww;
-    WCK wc;
-    JRK jr;
-    KurK kur;
-    RWWExK rwwex;
+template <class T>
+struct WCKt { T dt, sqrt_dt, itau_E, itau_I, a_E, a_I, mu_E, mu_I; };
+template <class T>
+struct JRKt { T dt, sqrt_dt, A, B, a, b, v0, nu_max, r, mu, cmin, cmax, midpoint, a_sq, b_sq; };
+template <class T>
+struct KurKt { T dt, sqrt_dt, twopi; };
+template <class T>
+struct RWWExKt { T dt, sqrt_dt, J_N, a, b, d, dt_itau, dt_gamma; };
+using RWWK = RWWKt<double>;
+using WCK = WCKt<double>;
+using JRK = JRKt<double>;
+using KurK = KurKt<double>;
+using RWWExK = RWWExKt<double>;
+template <class T>
+union ModelKt {
+    RWWKt<T> rww;
+    WCKt<T> wc;
+    JRKt<T> jr;
+    KurKt<T> kur;
+    RWWExKt<T> rwwex;
+    T all[24];   // the members of one model in order
 };
+using ModelK = ModelKt<double>;
+using ModelKf = ModelKt<float>;
+static_assert(sizeof(ModelK) == 24 * sizeof(double) && sizeof(ModelKf) == 24 * sizeof(float), "constants");
 
 // Static description of each model (include/cubnm/models/<model>.hpp).
 struct ModelDesc {
@@ -95,6 +111,7 @@ struct IntegrateArgs {
     double init_delta;
     BWConst bw;
     ModelK K;
+    ModelKf Kf;                  // K rounded to float
     int sim_begin;               // first simulation of this launch (FP64 kernel)
     int n_regional;              // regional parameters of the model
     const int *tiles;            // FP32 kernel: [n_tiles][1 + tile_width] = SC index, then simulation ids (-1 = empty)
@@ -126,6 +143,24 @@ struct IntegrateArgs {
     int ell_tables;              // delay tables packed per SC (1 without delays)
     const int2 *ell_pk32;        // [n_scs][ell_tables][ell_k][nodes] {offset, float weight bits} (FP32 kernel)
     const int4 *ell_pk64;        // [n_scs][ell_tables][ell_k][nodes] {weight lo, weight hi, offset, 0} (FP64 kernel)
+    // Delay kernel (integrate_delay.cuh; lists from delay_plan.h), per used (SC, delay
+    // table) pair.  Ring buffers [CTA][node][db_window] in hist / hist_f32.
+    int db_window;               // slots per node: the largest delay rounded up to 32
+    int db_tiles, db_tile_src;   // source tiles, and sources per tile
+    int db_bufs;                 // tile buffers in shared memory (2: the next tile loads during this one)
+    int db_blob_max;             // bytes reserved for a tile's entry lists in a buffer
+    int db_buf_bytes;            // bytes of a buffer (entry lists, then windows)
+    int db_buf_at;               // shared-memory offset of the buffers
+    int db_noise_steps;          // steps of noise the buffers hold (at most 32)
+    const int *db_pair;          // [n_sims] pair of each simulation
+    const int *db_blob_at;       // [n_pairs][db_tiles + 1] start of each tile's lists, in 16 bytes
+    const void *db_blob;         // entry lists (delay_plan.h)
+    int db_near_k;               // entries per near list (the longest of any pair)
+    const int *db_near;          // [n_pairs][db_near_k][nodes] near: source * 32 + delay (0: padding)
+    const float *db_near_w32;
+    const double *db_near_w64;
+    const int *db_near_cnt;      // [n_pairs] longest near list of the pair
+    const int *db_near_min;      // [n_pairs] smallest near delay of the pair (32 if none)
 };
 
 // FC / FCD (reference: src/ext/fc.cu, src/ext/fc.cpp).
@@ -154,6 +189,12 @@ struct GofArgs {
 // launchers (return cudaGetLastError() of the launch)
 cudaError_t launch_integrate_fp64(int model, const IntegrateArgs &a, cudaStream_t st);
 cudaError_t launch_integrate_fp32(int model, const IntegrateArgs &a, cudaStream_t st, int *launches);
+// Conduction delays, blocks of 32 steps (integrate_delay.cuh).
+struct DelayLaunch { int threads, grid; size_t smem; };
+cudaError_t delay_config64(int model, const IntegrateArgs &a, int sms, DelayLaunch *c);
+cudaError_t delay_config32(int model, const IntegrateArgs &a, int sms, DelayLaunch *c);
+cudaError_t launch_delay64(int model, const IntegrateArgs &a, const DelayLaunch &c, cudaStream_t st);
+cudaError_t launch_delay32(int model, const IntegrateArgs &a, const DelayLaunch &c, cudaStream_t st);
 cudaError_t launch_integrate_simt32(int model, const IntegrateArgs &a, cudaStream_t st);  // FP32, one CTA per simulation
 // FP32 with 16 simulations on the lanes (integrate_lanes.cu): delays and/or > 128 nodes.
 bool lanes_supported(int model, int nodes, bool numerical_fic);

@@ -8,6 +8,10 @@
 // functions of rWW / rWWEx use expm1 (x / (1 - e^{-dx}) loses all its digits to
 // cancellation near x = 0 in single precision).
 //
+// step() takes the constants in either width (ModelK, or ModelKf, their float
+// rounding, which the FP32 kernels read from the parameter space without a
+// conversion or a register each).
+//
 // State layout per model: s[NS] state variables (type S) in the reference's
 // order, iv[NI] intermediates (type R), r[NR] regional parameters (type P),
 // CONN = the state that couples, BOLDV = the one that drives the
@@ -22,18 +26,38 @@
 
 namespace cbnm {
 
-// x / (1 - exp(-d x)): rWW / rWWEx firing rate (rww.cpp:202-203, rwwex.cpp:62)
-template <class R>
-__device__ __forceinline__ R rate_of(R x, double d);
-template <>
-__device__ __forceinline__ double rate_of<double>(double x, double d) {
-    return x / (1 - exp(-d * x));
+// a / b by Newton's iteration on an approximate reciprocal and Markstein's final
+// residual correction (P. Markstein, IBM J. Res. Dev. 34, 1990), which rounds the
+// quotient of normal numbers correctly but for rare last-bit cases.  No branches, so
+// the divisions of a step overlap: the FP32 rWW step took 620 cycles of latency with
+// the operator's two, which serialise.  |b| must be neither 0, denormal nor above
+// 2^125 (FP32), 2^1021 (FP64).
+__device__ __forceinline__ float div_nr(float a, float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    r = fmaf(r, fmaf(-b, r, 1.0f), r);
+    const float q = a * r;
+    return fmaf(fmaf(-b, q, a), r, q);
 }
-template <>
-__device__ __forceinline__ float rate_of<float>(float x, double d) {
-    const float df = (float)d;
-    const float y = -df * x;
-    return (y == 0.0f) ? 1.0f / df : x / -expm1f(y);
+__device__ __forceinline__ double div_nr(double a, double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    r = fma(r, fma(-b, r, 1.0), r);
+    r = fma(r, fma(-b, r, 1.0), r);
+    const double q = a * r;
+    return fma(fma(-b, q, a), r, q);
+}
+
+// x / (1 - exp(-d x)): rWW / rWWEx firing rate (rww.cpp:202-203, rwwex.cpp:62).  The
+// exponent is capped where the rate is below 1e-29 (FP32) or 1e-300 (FP64) of x, so that
+// the divisor stays finite.
+__device__ __forceinline__ double rate_of(double x, double d) {
+    return div_nr(x, 1 - exp(fmin(-d * x, 690.0)));
+}
+__device__ __forceinline__ float rate_of(float x, float d) {
+    const float y = fminf(-d * x, 70.0f);
+    const bool zero = fabsf(y) < 1e-30f;   // the limit 1 / d, to rounding
+    return zero ? 1.0f / d : div_nr(x, zero ? 1.0f : -expm1f(y));
 }
 
 template <class R>
@@ -47,14 +71,15 @@ struct RWWm {
         s[4] = R(0.001); s[5] = R(0.001);
     }
     __device__ static void restart(S *s, R *, const P *) { s[4] = R(0.001); s[5] = R(0.001); }
-    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R n1, const ModelK &K) {  // rww.cpp:194-232
-        const RWWK &m = K.rww;
+    template <class KK>
+    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R n1, const KK &K) {  // rww.cpp:194-232
+        const auto &m = K.rww;
         s[0] = R(m.w_E__I_0) + r[0] * r[1] * s[4] + in * g[0] * r[1] - r[2] * s[5];
         s[1] = R(m.w_I__I_0) + r[1] * s[4] - R(m.w_II) * s[5];
         iv[0] = R(m.a_E) * s[0] - R(m.b_E);
         iv[1] = R(m.a_I) * s[1] - R(m.b_I);
-        s[2] = rate_of<R>(iv[0], m.d_E);
-        s[3] = rate_of<R>(iv[1], m.d_I);
+        s[2] = rate_of(iv[0], R(m.d_E));
+        s[3] = rate_of(iv[1], R(m.d_I));
         iv[2] = n0 * r[3] * R(m.sqrt_dt) + R(m.dt_gamma_E) * ((R(1) - s[4]) * s[2]) - R(m.dt_itau_E) * s[4];
         iv[3] = n1 * r[3] * R(m.sqrt_dt) + R(m.dt_gamma_I) * s[3] - R(m.dt_itau_I) * s[5];
         s[4] += iv[2];
@@ -72,8 +97,9 @@ struct WCm {
     static constexpr bool OSC = false, POSTBW = false;
     __device__ static void init(S *s, R *, const R *, const P *) { s[0] = R(0.001); s[1] = R(0.001); }
     __device__ static void restart(S *s, R *, const P *) { s[0] = R(0.001); s[1] = R(0.001); }
-    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R n1, const ModelK &K) {  // wc.cpp:51-80
-        const WCK &m = K.wc;
+    template <class KK>
+    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R n1, const KK &K) {  // wc.cpp:51-80
+        const auto &m = K.wc;
         iv[0] = R(1) / (R(1) + exp(-R(m.a_E) * (r[0] * s[0] - r[1] * s[1] + g[0] * in + r[4] - R(m.mu_E))));
         iv[1] = R(1) / (R(1) + exp(-R(m.a_I) * (r[2] * s[0] - r[3] * s[1] + r[5] - R(m.mu_I))));
         iv[2] = (-s[0] + (R(1) - s[0]) * iv[0]) * R(m.itau_E);
@@ -95,8 +121,9 @@ struct JRm {
         for (int i = 0; i < 8; ++i) s[i] = R(0);
     }
     __device__ static void restart(S *s, R *, const P *) { for (int i = 0; i < 8; ++i) s[i] = R(0); }
-    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const ModelK &K) {  // jr.cpp:80-133
-        const JRK &m = K.jr;
+    template <class KK>
+    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const KK &K) {  // jr.cpp:80-133
+        const auto &m = K.jr;
         iv[0] = R(2) * R(m.nu_max) / (R(1) + exp(R(m.r) * (R(m.v0) - (s[1] - s[2]))));
         iv[1] = R(2) * R(m.nu_max) / (R(1) + exp(R(m.r) * (R(m.v0) - (r[1] * r[0] * s[0]))));
         iv[2] = R(2) * R(m.nu_max) / (R(1) + exp(R(m.r) * (R(m.v0) - (r[3] * r[0] * s[0]))));
@@ -125,8 +152,9 @@ struct Kuramotom {
     static constexpr bool OSC = true, POSTBW = false;
     __device__ static void init(S *s, R *, const R *, const P *r) { s[0] = S(r[0]); }
     __device__ static void restart(S *s, R *, const P *r) { s[0] = S(r[0]); }
-    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const ModelK &K) {  // kuramoto.cpp:48-61
-        const KurK &m = K.kur;
+    template <class KK>
+    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const KK &K) {  // kuramoto.cpp:48-61
+        const auto &m = K.kur;
         const S w = r[1] + S(g[0] * in);  // instantaneous frequency, in double
         iv[0] = R(w);
         s[0] = s[0] + m.dt * w + m.sqrt_dt * S(n0) * r[2];
@@ -142,11 +170,12 @@ struct RWWExm {
     static constexpr bool OSC = false, POSTBW = false;
     __device__ static void init(S *s, R *, const R *, const P *) { s[0] = s[1] = R(0); s[2] = R(0.001); }
     __device__ static void restart(S *s, R *, const P *) { s[2] = R(0.001); }
-    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const ModelK &K) {  // rwwex.cpp:48-73
-        const RWWExK &m = K.rwwex;
+    template <class KK>
+    __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const KK &K) {  // rwwex.cpp:48-73
+        const auto &m = K.rwwex;
         s[0] = r[0] * R(m.J_N) * s[2] + g[0] * R(m.J_N) * in + r[1];
         iv[0] = R(m.a) * s[0] - R(m.b);
-        s[1] = rate_of<R>(iv[0], m.d);
+        s[1] = rate_of(iv[0], R(m.d));
         iv[1] = R(m.dt_gamma) * ((R(1) - s[2]) * s[1]) - R(m.dt_itau) * s[2] + n0 * R(m.sqrt_dt) * r[2];
         s[2] += iv[1];
         s[2] = fmax(R(0), fmin(R(1), s[2]));

@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/cubnm_b200.h"
+#include "delay_plan.h"
 #include "engine.h"
 #include "tc_common.cuh"
 
@@ -328,6 +329,7 @@ struct Session {
     DBuf d_bold, d_states, d_gbools, d_gints, d_fc, d_fcd, d_wfc, d_pairs_i, d_pairs_j, d_wstart, d_wend, d_status;
     DBuf d_tiles, d_sct_f32, d_ell_pk, d_bw_scr, d_ln_groups, d_ln_params, d_ln_hist, d_ln_bw;
     DBuf fl_ec, fl_q, fl_win, fl_scr;  // fit loss
+    DBuf d_db_pair, d_db_at, d_db_blob, d_db_near, d_db_near_w, d_db_near_n;  // delay kernel lists
     DBuf d_pidx, d_wstat;              // tensor-core FC: pair index of (i, j); window-FC statistics
     // gof
     DBuf g_simfc, g_empfc, g_simfcd, g_empfcd, g_out;
@@ -383,6 +385,7 @@ static void close_session(Session *&p) {
                         &S.d_hist, &S.d_hist_f32, &S.d_bold, &S.d_states, &S.d_gbools, &S.d_gints, &S.d_fc,
                         &S.d_fcd, &S.d_wfc, &S.d_pairs_i, &S.d_pairs_j, &S.d_wstart, &S.d_wend, &S.d_status, &S.d_tiles,
                         &S.d_sct_f32, &S.d_ell_pk, &S.d_bw_scr, &S.d_ln_groups, &S.d_ln_params, &S.d_ln_hist, &S.d_ln_bw, &S.fl_ec, &S.fl_q, &S.fl_win, &S.fl_scr, &S.d_pidx, &S.d_wstat,
+                        &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
                         &S.g_simfc, &S.g_empfc, &S.g_simfcd, &S.g_empfcd, &S.g_out})
             b->release();
         for (auto &ev : S.ev) cudaEventDestroy(ev);
@@ -915,13 +918,13 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         has_delay = *std::max_element(h_max_delay.begin(), h_max_delay.end()) > 0;
     }
     // FP32 kernels: the tensor-core tiles take shared-SC batches without delays or
-    // numerical FIC at <= 128 nodes.  Delayed networks of more than 512 nodes, with
-    // at least half as many 16-simulation groups as SMs, take the lane kernel
-    // (1,000-node WC, 2,048 sims: 440 vs 343 sims x sim-s / s); everything else runs
-    // on the per-simulation kernel, which measured faster there (400-node rWW with
-    // delays: 1,103 vs 435; 200-node rWW without, 512 sims: 11,645 vs 1,593).  The
-    // lane kernel also runs the G tangent, and when CBNM_FP32_KERNEL=lanes or the
-    // tuner picks it; CBNM_FP32_KERNEL=simt forces the per-simulation kernel.
+    // numerical FIC at <= 128 nodes; delayed networks run in blocks of 32 steps
+    // (integrate_delay.cuh: 1,000-node WC, 148 sims: 31,000 cycles per sim-step and SM
+    // against the lane kernel's 66,000), everything else on the per-simulation kernel
+    // (200-node rWW without delays, 512 sims: 11,645 sims x sim-s / s against the lane
+    // kernel's 1,593).  The lane kernel runs the G tangent, and when
+    // CBNM_FP32_KERNEL=lanes or the tuner picks it; CBNM_FP32_KERNEL=simt forces the
+    // per-simulation kernel.
     const char *fp32_kernel = std::getenv("CBNM_FP32_KERNEL");
     const bool force_simt = fp32_kernel && std::string(fp32_kernel) == "simt";
     const bool force_lanes = fp32_kernel && std::string(fp32_kernel) == "lanes";
@@ -961,15 +964,40 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     }
     const bool use_tc = variant == V_DEFAULT ? (!tan_bold && !force_simt && tc_ok)
                                              : (variant == V_PP || variant == V_PPWS || variant == V_V5);
-    const bool lanes_default = has_delay && n > 512 && 2 * ((N + 15) / 16) >= sm_count() && !force_simt;
-    bool use_lanes = variant == V_DEFAULT ? (lanes_ok && (tan_bold || ((force_lanes || lanes_default) && !use_tc)))
+    bool use_lanes = variant == V_DEFAULT ? (lanes_ok && (tan_bold || (force_lanes && !use_tc)))
                                           : (variant == V_LANES || variant == V_LANES512);
     const int lanes_threads = variant == V_LANES512 ? 512 : 1024;
     if (t_round && !t_round_resolved && !(use_lanes && lanes_threads == 1024 && !tan_bold && g_batch_launch)) {
         t_round_resolved = true;  // this group runs its own integrator: the round need not wait for it
         round_decline(*t_round);
     }
-    if (has_delay) {
+    // Delayed networks run in blocks of 32 steps (integrate_delay.cuh) unless a kernel
+    // or coupling form is forced; the phase model, whose coupling depends on the
+    // target's current phase, keeps the per-step loop, as do networks of which most
+    // delays are below a block, and FP64 networks whose rows do not fit shared memory.
+    DelayPlan plan;
+    bool delay_blocks = has_delay && !md.osc && !use_lanes && !force_simt && !std::getenv("CBNM_COUPLING");
+    const double *sc_host = h_sc;
+    std::vector<double> sc_copy;
+    if (has_delay && device_io) {
+        sc_copy.resize(nn * a->n_scs);
+        CK(cudaMemcpy(sc_copy.data(), a->sc, sizeof(double) * sc_copy.size(), cudaMemcpyDeviceToHost));
+        sc_host = sc_copy.data();
+        if (h_sc_idx.size() != (size_t)N) {
+            h_sc_idx.resize(N);
+            CK(cudaMemcpy(h_sc_idx.data(), a->sc_indices, sizeof(int) * N, cudaMemcpyDeviceToHost));
+        }
+    }
+    if (delay_blocks) {
+        const int *sc_of = device_io ? h_sc_idx.data() : a->sc_indices;
+        const int dmax = *std::max_element(h_max_delay.begin(), h_max_delay.end());
+        const size_t most = (size_t)1 << 30;
+        delay_blocks = c.fp32 ? build_delay_plan<float>(plan, n, N, md.n_noise, sm_count(), sc_host, sc_of, h_delay,
+                                                        h_delay_idx, dmax, most)
+                              : build_delay_plan<double>(plan, n, N, md.n_noise, sm_count(), sc_host, sc_of, h_delay,
+                                                         h_delay_idx, dmax, most);
+    }
+    if (has_delay && !delay_blocks) {
         S.d_delay.ensure(sizeof(int) * h_delay.size());
         CK(cudaMemcpyAsync(S.d_delay.p, h_delay.data(), sizeof(int) * h_delay.size(), cudaMemcpyHostToDevice, S.st));
         S.d_delay_idx.ensure(sizeof(int) * N);
@@ -1036,6 +1064,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         }
     }
     ia.K = make_constants(md.id, c.dt);
+    for (int i = 0; i < 24; ++i) ia.Kf.all[i] = (float)ia.K.all[i];
     {  // the two-tile kernel reads these from its parameter space
         BWFast &f = ia.bwf;
         f.dt = ia.bw.dt; f.kappa = ia.bw.kappa; f.y = ia.bw.y; f.dt_itau = ia.bw.dt_itau; f.ialpha = ia.bw.ialpha;
@@ -1067,7 +1096,42 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         CK(cudaMemcpyAsync(S.d_sc_f32.p, f.data(), sizeof(float) * f.size(), cudaMemcpyHostToDevice, S.st));
         ia.sc_f32 = S.d_sc_f32.as<float>();
     }
-    if (!use_tc) {
+    DelayLaunch dl{};
+    if (delay_blocks) {
+        auto up = [&](DBuf &b, const void *p, size_t bytes) {
+            b.ensure(bytes);
+            CK(cudaMemcpyAsync(b.p, p, bytes, cudaMemcpyHostToDevice, S.st));
+        };
+        up(S.d_db_pair, plan.pair.data(), sizeof(int) * plan.pair.size());
+        up(S.d_db_at, plan.blob_at.data(), sizeof(int) * plan.blob_at.size());
+        up(S.d_db_blob, plan.blob.data(), plan.blob.size());
+        up(S.d_db_near, plan.near.data(), sizeof(int) * plan.near.size());
+        std::vector<int> nearn(plan.near_cnt);
+        nearn.insert(nearn.end(), plan.near_min.begin(), plan.near_min.end());
+        up(S.d_db_near_n, nearn.data(), sizeof(int) * nearn.size());
+        const std::vector<float> near_w32(plan.near_w.begin(), plan.near_w.end());   // weights in the run's precision
+        if (c.fp32) up(S.d_db_near_w, near_w32.data(), sizeof(float) * near_w32.size());
+        else up(S.d_db_near_w, plan.near_w.data(), sizeof(double) * plan.near_w.size());
+        ia.db_window = plan.window; ia.db_tiles = plan.tiles; ia.db_tile_src = plan.tile_src; ia.db_bufs = plan.bufs;
+        ia.db_blob_max = plan.blob_max; ia.db_buf_bytes = plan.buf_bytes; ia.db_buf_at = plan.buf_at;
+        ia.db_noise_steps = plan.noise_steps;
+        ia.db_pair = S.d_db_pair.as<int>(); ia.db_blob_at = S.d_db_at.as<int>(); ia.db_blob = S.d_db_blob.p;
+        ia.db_near_k = plan.near_k; ia.db_near = S.d_db_near.as<int>();
+        ia.db_near_cnt = S.d_db_near_n.as<int>(); ia.db_near_min = S.d_db_near_n.as<int>() + plan.n_pairs;
+        dl.threads = plan.threads;
+        dl.smem = plan.smem;
+        CK((c.fp32 ? delay_config32 : delay_config64)(md.id, ia, sm_count(), &dl));
+        const size_t slots = (size_t)n * plan.window * dl.grid;
+        if (c.fp32) {
+            ia.db_near_w32 = S.d_db_near_w.as<float>();
+            ia.hist_f32 = (float *)S.d_hist_f32.ensure(sizeof(float) * slots);
+        } else {
+            ia.db_near_w64 = S.d_db_near_w.as<double>();
+            ia.hist = (double *)S.d_hist.ensure(sizeof(double) * slots);
+        }
+        CK(cudaStreamSynchronize(S.st));  // host vectors go out of scope
+    }
+    if (!use_tc && !delay_blocks) {
         // Sparse coupling for the per-simulation kernels (ELLPACK by target node):
         // used when the densest column of every SC holds at most half the nodes
         // (CBNM_COUPLING=sparse|dense overrides).  Zero weights are skipped and the
@@ -1250,6 +1314,10 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
             CK(launch_integrate_lanes(md.id, ia, S.st));
             launches += 2;  // parameter layout + integrator
         }
+    } else if (delay_blocks) {
+        CK(cudaEventRecord(S.ev[1], S.st));
+        CK((c.fp32 ? launch_delay32 : launch_delay64)(md.id, ia, dl, S.st));
+        ++launches;
     } else if (c.fp32) {
         CK(cudaStreamSynchronize(S.st));
         CK(cudaEventRecord(S.ev[1], S.st));
@@ -1452,6 +1520,7 @@ static AdjArgs adjoint_args(Session &S, AdjPlan &P, const cbnm_run_args *a) {
     ia.noise_f32 = S.d_noise_f32.as<float>(); ia.sh_nodes = S.d_sh_nodes.as<int>(); ia.sh_ts = S.d_sh_ts.as<int>();
     ia.bw = g_bw; ia.bw.dt = c.bw_dt; ia.bw.dt_itau = ia.bw.dt * ia.bw.itau;  // core.cpp:291-292
     ia.K = make_constants(MODEL_RWW, c.dt);
+    for (int i = 0; i < 24; ++i) ia.Kf.all[i] = (float)ia.K.all[i];
     A.sct_f32 = S.d_sct_f32.as<float>();
     A.seg_bw = P.seg_bw; A.n_seg = P.n_seg;
     return A;

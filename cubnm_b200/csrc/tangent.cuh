@@ -50,7 +50,7 @@ struct Tangent<RWWm<float>> {
         const float IE = float(m.w_E__I_0) + r[0] * r[1] * SE + in * g[0] * r[1] - r[2] * SI;
         const float II = float(m.w_I__I_0) + r[1] * SE - float(m.w_II) * SI;
         const float xE = float(m.a_E) * IE - float(m.b_E), xI = float(m.a_I) * II - float(m.b_I);
-        const float rE = rate_of<float>(xE, m.d_E), rI = rate_of<float>(xI, m.d_I);
+        const float rE = rate_of(xE, (float)m.d_E), rI = rate_of(xI, (float)m.d_I);
         const float dIE = r[0] * r[1] * dSE + r[1] * (in + g[0] * din) - r[2] * dSI;
         const float dII = r[1] * dSE - float(m.w_II) * dSI;
         const float drE = rate_deriv_f(xE, float(m.d_E)) * float(m.a_E) * dIE;
