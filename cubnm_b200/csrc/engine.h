@@ -114,12 +114,10 @@ struct IntegrateArgs {
     ModelKf Kf;                  // K rounded to float
     int sim_begin;               // first simulation of this launch (FP64 kernel)
     int n_regional;              // regional parameters of the model
-    const int *tiles;            // FP32 kernel: [n_tiles][1 + tile_width] = SC index, then simulation ids (-1 = empty)
+    const int *tiles;            // tile kernels: [n_tiles][1 + width] = SC index, then simulation ids (-1 = empty)
     int n_tiles;
-    int tile_width;              // FP32 kernel: simulations per tile (16 or 32)
-    double bw_binom[13];         // FP32 kernel: binomial coefficients C(1/alpha, k), k = 0..12
-    BWFast bwf;                  // two-tile kernel: Balloon-Windkessel constants
-    alignas(8) float k32[24];    // two-tile kernel: the model's FP32 constants (M::K)
+    BWFast bwf;                  // Balloon-Windkessel constants of the series form
+    alignas(8) float k32[24];    // tensor-core kernels: the model's FP32 constants (M::K)
     int *status;                 // device status word (0 = ok)
     double *bw_scratch;          // two-tile kernel: per-CTA Balloon-Windkessel state (pp_bw_scratch_bytes)
     int pp_grid;                 // two-tile kernel: CTAs launched (the scratch holds this many)
@@ -188,7 +186,20 @@ struct GofArgs {
 
 // launchers (return cudaGetLastError() of the launch)
 cudaError_t launch_integrate_fp64(int model, const IntegrateArgs &a, cudaStream_t st);
-cudaError_t launch_integrate_fp32(int model, const IntegrateArgs &a, cudaStream_t st, int *launches);
+// FP32, eight simulations of one SC per CTA on warp-level matrix products (integrate_mma.cu).
+// Tiles: [n_tiles][1 + FP32_TILE] = SC index, then simulation ids (-1 = empty).
+constexpr int FP32_TILE = 8;
+// FP32, 32 simulations of one SC per CTA on tcgen05 (integrate_fp32.cu): large batches, <= 128 nodes.
+constexpr int FP32_TILE_TC = 32;
+bool tc32_supported(int model, int nodes);
+cudaError_t launch_integrate_tc32(int model, const IntegrateArgs &a, cudaStream_t st);
+cudaError_t launch_integrate_mma(int model, const IntegrateArgs &a, cudaStream_t st);
+// FP64, no delays, up to 128 nodes (integrate_tile64.cu): tiles of eight simulations of one
+// SC where a.tiles is set (laid out as above), else one simulation per CTA.
+constexpr int FP64_TILE = 8;
+bool tile64_supported(int model, int nodes);
+cudaError_t launch_integrate_tile64(int model, const IntegrateArgs &a, cudaStream_t st);
+void fill_k32(int model, const ModelK &K, float *k32);   // the model's FP32 constants
 // Conduction delays, blocks of 32 steps (integrate_delay.cuh).
 struct DelayLaunch { int threads, grid; size_t smem; };
 cudaError_t delay_config64(int model, const IntegrateArgs &a, int sms, DelayLaunch *c);
@@ -214,7 +225,6 @@ bool fp32_supported(int model, int nodes, bool has_delay);
 bool pp_supported(int model, int nodes, bool has_delay);
 size_t pp_bw_scratch_bytes(int nodes, int grid);
 cudaError_t launch_integrate_pp(int model, const IntegrateArgs &a, cudaStream_t st, int *launches);
-int fp32_tile_for(int nodes);  // simulations per FP32 tile for a node count
 // rWW analytical FIC (fic.cu): wIE written into regional row 2 in place.
 struct FicArgs {
     int nodes, n_sims;

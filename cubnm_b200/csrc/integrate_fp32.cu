@@ -3,11 +3,9 @@
 // The same time loop as the FP64 kernel (reference: src/ext/bnm.cu:117-505),
 // reorganised for B200:
 //
-//  * A CTA integrates a tile of TN simulations that share one SC (TN = 16 with
-//    two CTAs per SM, or 32 with one).  Node j of the tile lives on TMEM lane j
-//    (M = 128 lanes, nodes <= 128); each thread owns one node and SPT
-//    simulations (4 in the 16-wide tile, 8 in the 32-wide one); warpgroup g
-//    owns simulations [SPT g, SPT g + SPT) of the tile.
+//  * A CTA integrates a tile of TN = 32 simulations that share one SC.  Node j of
+//    the tile lives on TMEM lane j (M = 128 lanes, nodes <= 128); each thread owns
+//    one node and SPT = 8 simulations; warpgroup g owns simulations [8 g, 8 g + 8).
 //  * Coupling (bnm.cu:48-77) is a GEMM every step:
 //        D[j][s] = sum_k SC[k][j] * x_k^s
 //    issued as tcgen05.mma kind::f16 with A = SC^T held in TMEM (BF16, written
@@ -17,15 +15,22 @@
 //    (lane 0 of warps 0..2) into three accumulator sets that the readers add:
 //    one thread issuing all 21 MMAs of a step was itself a bottleneck (the
 //    three-issuer form measured 8% faster; a fourth issuer no further gain, as
-//    the tensor pipe then bounds the GEMM).  Keeping A in TMEM leaves only the 16-column x
-//    slice to be read from shared memory per MMA.  Elementwise model updates run
+//    the tensor pipe then bounds the GEMM; x hi and x lo side by side in one MMA of N = 64,
+//    14 MMAs instead of 21, measured 8% slower).  Keeping A in TMEM leaves only x to be
+//    read from shared memory per MMA.  Elementwise model updates run
 //    in FP32 registers.
 //  * The Balloon-Windkessel state (bnm.cu:357-371) stays FP64 and lives in TMEM
 //    (8 x 32-bit words per simulation).  The update of bw step m runs during the
 //    GEMMs of bw step m+1 (one simulation pair per inner step), from the inputs
-//    saved at the end of step m, so the FP64 work overlaps the tensor core.
+//    saved at the end of step m, so the FP64 work overlaps the tensor core.  The pair's
+//    two chains overlap (bw_step64_n: 5,172 -> 4,793 cycles a step at 100 nodes); one
+//    simulation per inner step instead of a pair measured 6,180.
 //  * Every wait on the MMA barrier is bounded; on timeout the CTA records a
 //    status, leaves its loop, frees its TMEM and returns.
+//
+// This is the form for large batches; up to 16 simulations per SM integrate_mma.cu's
+// eight-wide tiles are faster (100 nodes, cycles a step of the whole batch: 512 sims
+// 1,900 against 5,172; 2,368 sims 2,650; 4,736 sims 5,250 against 4,793 here).
 //
 // TMEM columns: [0, NACC TN) accumulator sets | [NACC TN, NACC TN + KP) SC^T hi then lo, two BF16
 // per column, K chunk kk at +8kk | [COLS - 8 TN, COLS) Balloon-Windkessel state.
@@ -34,7 +39,6 @@
 //   LBO_B = TN/8 * 128 B (K-direction core-matrix stride), SBO = 128 B.
 #include <algorithm>
 #include <cstdint>
-#include <cstdlib>
 #include <cuda_bf16.h>
 #include "engine.h"
 #include "tc_common.cuh"
@@ -44,22 +48,12 @@ namespace {
 
 constexpr int COL_ACC = 0;           // accumulator columns start here
 
-// Tile geometry: TN simulations per tile (MMA N), SPT simulations per thread,
-// TN/SPT warpgroups per CTA.
-template <int TN_, int SPT_, int NACC_>
-struct Tile {
-    static constexpr int TN = TN_;
-    static constexpr int SPT = SPT_;
-    static constexpr int NACC = NACC_;   // independent accumulator sets the GEMM round-robins over
-    static constexpr int NWG = TN / SPT;
-    static constexpr int NTHREADS = NWG * 128;
-    static constexpr int TMEM_COLS = TN >= 32 ? 512 : 256;   // one CTA an SM at 32 wide, two at 16
-    static constexpr int CTAS_PER_SM = 512 / TMEM_COLS;
-    static constexpr uint32_t LBO_B = (TN / 8) * 128;
-    // threads that issue the step's GEMM: 1 (all MMAs, round-robin over the NACC sets)
-    // or NACC (thread p of warp p issues pass p of BF16x3 into accumulator set p)
-    static constexpr int ISSUERS = (NACC == 3) ? 3 : 1;
-};
+constexpr int TN = 32;                 // simulations per tile (MMA N)
+constexpr int SPT = 8;                 // of which each thread owns SPT
+constexpr int NACC = 3;                // accumulator sets: thread 0 of warp p issues BF16x3 pass p into set p
+constexpr int NTHREADS = TN / SPT * 128;
+constexpr int TMEM_COLS = 512;         // one CTA an SM
+constexpr uint32_t LBO_B = (TN / 8) * 128;
 
 struct Smem {
     uint64_t mbar;
@@ -69,13 +63,8 @@ struct Smem {
 };
 
 // ---------------------------------------------------------------- kernel
-template <class M, class T>
-__global__ void __launch_bounds__(T::NTHREADS, T::CTAS_PER_SM) k_integrate_tc(const IntegrateArgs a, const int *tiles,
-                                                                              int n_tiles, int KP) {
-    constexpr int TN = T::TN, TMEM_COLS = T::TMEM_COLS;
-    constexpr uint32_t LBO_B = T::LBO_B;
-    constexpr int NACC = T::NACC;
-    constexpr int SPT = T::SPT;
+template <class M>
+__global__ void __launch_bounds__(NTHREADS, 1) k_integrate_tc(const IntegrateArgs a, const int *tiles, int n_tiles, int KP) {
     constexpr int COL_A = TN * NACC;                   // A_hi at COL_A, A_lo at COL_A + KP/2 (bf16 pairs)
     constexpr int COL_BWT = TMEM_COLS - TN * 8;        // Balloon-Windkessel state at the top
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -100,8 +89,8 @@ __global__ void __launch_bounds__(T::NTHREADS, T::CTAS_PER_SM) k_integrate_tc(co
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        // one arrival per issuing thread (ISSUERS of them commit each step)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm->mbar)), "r"(T::ISSUERS));
+        // one arrival per issuing thread (NACC of them commit each step)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm->mbar)), "r"(NACC));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         sm->abort = 0;
         sm->sc_loaded = -1;
@@ -195,13 +184,8 @@ __global__ void __launch_bounds__(T::NTHREADS, T::CTAS_PER_SM) k_integrate_tc(co
             // simulations n = wg*SPT .. wg*SPT+SPT-1 of the tile
             const int n0 = wg * SPT;
             const uint32_t off = (j >> 3) * LBO_B + (n0 >> 3) * 128 + (j & 7) * 16 + (n0 & 7) * 2;
-            if constexpr (SPT == 8) {
-                *reinterpret_cast<uint4 *>(B_hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                *reinterpret_cast<uint4 *>(B_lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-            } else {
-                *reinterpret_cast<uint2 *>(B_hi + off) = make_uint2(hw[0], hw[1]);
-                *reinterpret_cast<uint2 *>(B_lo + off) = make_uint2(lw[0], lw[1]);
-            }
+            *reinterpret_cast<uint4 *>(B_hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            *reinterpret_cast<uint4 *>(B_lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         };
         write_x();
         if (tid == 0) sm->sc_loaded = sc_idx;
@@ -267,42 +251,18 @@ __global__ void __launch_bounds__(T::NTHREADS, T::CTAS_PER_SM) k_integrate_tc(co
                 __syncthreads();
                 if (sm->abort) { aborted = true; break; }
                 // (2) the BF16x3 coupling GEMM (A from TMEM, B from SMEM)
-                if constexpr (T::ISSUERS == 3) {
-                    // three issuing threads in three warps, one BF16x3 pass each, into
-                    // accumulator sets 0..2; each commits its own MMAs to the barrier
-                    if ((tid & 31) == 0 && warp < 3) {
-                        fence_after();
-                        const int pass = warp;
-                        const uint32_t bh = smem_u32(B_hi), bl = smem_u32(B_lo);
-                        const uint32_t d = tmem + COL_ACC + pass * TN;
-                        const int nk = KP / 16;
-                        for (int kk = 0; kk < nk; ++kk) {
-                            const uint32_t ta = tmem + COL_A + (pass == 2 ? half : 0) + kk * 8;
-                            const uint64_t db = smem_desc((pass == 1 ? bl : bh) + kk * 2 * LBO_B, LBO_B, 128);
-                            mma_bf16_ts(d, ta, db, idesc, kk > 0 ? 1u : 0u);
-                        }
-                        mma_commit(mbar);
-                    }
-                } else if (tid == 0) {
+                // three issuing threads in three warps, one BF16x3 pass each, into
+                // accumulator sets 0..2; each commits its own MMAs to the barrier
+                if ((tid & 31) == 0 && warp < NACC) {
                     fence_after();
+                    const int pass = warp;
                     const uint32_t bh = smem_u32(B_hi), bl = smem_u32(B_lo);
+                    const uint32_t d = tmem + COL_ACC + pass * TN;
                     const int nk = KP / 16;
-                    // consecutive MMAs go to different accumulator sets so they do not
-                    // wait on each other's read-modify-write of the same TMEM columns
-                    int issued = 0;
                     for (int kk = 0; kk < nk; ++kk) {
-                        const uint32_t tah = tmem + COL_A + kk * 8, tal = tmem + COL_A + half + kk * 8;
-                        const uint64_t dbh = smem_desc(bh + kk * 2 * LBO_B, LBO_B, 128);
-                        const uint64_t dbl = smem_desc(bl + kk * 2 * LBO_B, LBO_B, 128);
-#pragma unroll
-                        for (int pass = 0; pass < 3; ++pass, ++issued) {
-                            const int set = issued % NACC;
-                            const uint32_t d = tmem + COL_ACC + set * TN;
-                            const uint32_t accumulate = issued >= NACC ? 1u : 0u;
-                            if (pass == 0) mma_bf16_ts(d, tah, dbh, idesc, accumulate);
-                            else if (pass == 1) mma_bf16_ts(d, tah, dbl, idesc, accumulate);
-                            else mma_bf16_ts(d, tal, dbh, idesc, accumulate);
-                        }
+                        const uint32_t ta = tmem + COL_A + (pass == 2 ? half : 0) + kk * 8;
+                        const uint64_t db = smem_desc((pass == 1 ? bl : bh) + kk * 2 * LBO_B, LBO_B, 128);
+                        mma_bf16_ts(d, ta, db, idesc, kk > 0 ? 1u : 0u);
                     }
                     mma_commit(mbar);
                 }
@@ -408,64 +368,33 @@ __global__ void __launch_bounds__(T::NTHREADS, T::CTAS_PER_SM) k_integrate_tc(co
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-using Tile16 = Tile<16, 8, 1>;   // 2 warpgroups x 8 simulations, two CTAs per SM
-using Tile32 = Tile<32, 8, 3>;   // 4 warpgroups x 8 simulations, one CTA per SM, 3 GEMM issuers
-
-template <class T>
-size_t smem_bytes(int KP) { return (size_t)2 * KP * T::TN * 2 + sizeof(Smem) + 64; }
+size_t smem_bytes(int KP) { return (size_t)2 * KP * TN * 2 + sizeof(Smem) + 64; }
 // the time-averaged state sums [NOUT][TN][nodes] (FP32)
-template <class M, class T>
-size_t sacc_bytes(int nodes) { return sizeof(float) * (size_t)M::NOUT * T::TN * nodes + 16; }
+template <class M>
+size_t sacc_bytes(int nodes) { return sizeof(float) * (size_t)M::NOUT * TN * nodes + 16; }
 
-template <class M, class T>
-cudaError_t launch_tc(const IntegrateArgs &a, const int *tiles, int n_tiles, cudaStream_t st) {
+template <class M>
+cudaError_t launch_model(const IntegrateArgs &a, cudaStream_t st) {
     const int KP = ((a.nodes + 15) / 16) * 16;
-    // shared memory large enough that no more CTAs than TMEM holds land on one SM
-    const size_t floor = T::CTAS_PER_SM == 2 ? 80 * 1024 : 120 * 1024;
-    const size_t smem = std::max<size_t>(smem_bytes<T>(KP) + sacc_bytes<M, T>(a.nodes), floor);
-    cudaError_t e = allow_dynamic_smem(k_integrate_tc<M, T>);
+    // shared memory large enough that one CTA lands on an SM (its TMEM is taken)
+    const size_t smem = std::max<size_t>(smem_bytes(KP) + sacc_bytes<M>(a.nodes), 120 * 1024);
+    cudaError_t e = allow_dynamic_smem(k_integrate_tc<M>);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = std::min(n_tiles, T::CTAS_PER_SM * sms);
-    k_integrate_tc<M, T><<<grid, T::NTHREADS, smem, st>>>(a, tiles, n_tiles, KP);
+    k_integrate_tc<M><<<std::min(a.n_tiles, sms), NTHREADS, smem, st>>>(a, a.tiles, a.n_tiles, KP);
     return cudaGetLastError();
 }
 
-template <class M>
-cudaError_t launch_model(const IntegrateArgs &a, cudaStream_t st) {
-    if (a.tile_width == 32) return launch_tc<M, Tile32>(a, a.tiles, a.n_tiles, st);
-    if (a.tile_width == 16) return launch_tc<M, Tile16>(a, a.tiles, a.n_tiles, st);
-    return cudaErrorInvalidValue;
-}
-
-// TMEM columns used: accumulator sets (NACC TN) + SC^T hi/lo (KP) + Balloon-Windkessel state (8 TN)
-template <class T>
-constexpr bool tmem_fits(int KP) { return T::NACC * T::TN + KP + 8 * T::TN <= T::TMEM_COLS; }
-
 }  // namespace
 
-// Tile width: 32 simulations (one CTA per SM, one 32-wide GEMM per step: the
-// tensor core's cost is per instruction at these widths, so the wider GEMM
-// halves it per simulation; measured 145k vs 140k sims*s/s for the 16-wide,
-// two-CTA form on the 100-node workload).  CBNM_FP32_TILE=16 selects the
-// 16-wide form where SC^T fits beside its state (nodes <= 112).
-int fp32_tile_for(int nodes) {
-    const char *e = std::getenv("CBNM_FP32_TILE");
-    const int KP = ((nodes + 15) / 16) * 16;
-    if (e && std::atoi(e) == 16 && tmem_fits<Tile16>(KP)) return 16;
-    return 32;
+// TMEM: accumulators (3 TN) + SC^T hi/lo (KP) + Balloon-Windkessel state (8 TN) fit up to 128 nodes.
+bool tc32_supported(int model, int nodes) {
+    return nodes <= TM && (model == MODEL_RWW || model == MODEL_WC || model == MODEL_JR || model == MODEL_RWWEX);
 }
 
-bool fp32_supported(int model, int nodes, bool has_delay) {
-    if (has_delay || nodes > TM || nodes < 1) return false;
-    if (!tmem_fits<Tile32>(((nodes + 15) / 16) * 16)) return false;
-    return model == MODEL_RWW || model == MODEL_WC || model == MODEL_JR || model == MODEL_RWWEX;
-}
-
-cudaError_t launch_integrate_fp32(int model, const IntegrateArgs &a, cudaStream_t st, int *launches) {
-    if (launches) ++*launches;
+cudaError_t launch_integrate_tc32(int model, const IntegrateArgs &a, cudaStream_t st) {
     switch (model) {
         case MODEL_RWW: return launch_model<RWW32>(a, st);
         case MODEL_WC: return launch_model<WC32>(a, st);

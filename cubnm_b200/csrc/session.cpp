@@ -78,6 +78,21 @@ static BWConst bw_defaults(double dt_s) {  // bw.cpp:4-22
 static BWConst g_bw = bw_defaults(0.001);
 static std::string g_err;
 
+// The Balloon-Windkessel constants of the series form, from ia.bw.
+static void fill_bwf(IntegrateArgs &ia) {
+    BWFast &f = ia.bwf;
+    f.dt = ia.bw.dt; f.kappa = ia.bw.kappa; f.y = ia.bw.y; f.dt_itau = ia.bw.dt_itau; f.ialpha = ia.bw.ialpha;
+    f.irho = 1.0 / ia.bw.rho; f.log2_omr = std::log2(ia.bw.oneminrho); f.ln_omr = std::log(ia.bw.oneminrho);
+    f.omr = ia.bw.oneminrho;
+    f.V0k1 = ia.bw.V_0 * ia.bw.k1; f.V0k2 = ia.bw.V_0 * ia.bw.k2; f.V0k3 = ia.bw.V_0 * ia.bw.k3;
+    long double v = 1.0L;   // C(1/alpha, k) for the binomial form of nu^(1/alpha)
+    f.binom[0] = 1.0;
+    for (int k = 1; k <= 12; ++k) {
+        v = v * ((long double)ia.bw.ialpha - (k - 1)) / k;
+        f.binom[k] = (double)v;
+    }
+}
+
 static ModelK make_constants(int model, double dt) {
     ModelK K;
     std::memset(&K, 0, sizeof(K));
@@ -918,11 +933,11 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         has_delay = *std::max_element(h_max_delay.begin(), h_max_delay.end()) > 0;
     }
     // FP32 kernels: the tensor-core tiles take shared-SC batches without delays or
-    // numerical FIC at <= 128 nodes; delayed networks run in blocks of 32 steps
-    // (integrate_delay.cuh: 1,000-node WC, 148 sims: 31,000 cycles per sim-step and SM
-    // against the lane kernel's 66,000), everything else on the per-simulation kernel
-    // (200-node rWW without delays, 512 sims: 11,645 sims x sim-s / s against the lane
-    // kernel's 1,593).  The lane kernel runs the G tangent, and when
+    // numerical FIC at <= 224 nodes (200-node rWW, 512 sims: 3,150 cycles a step of the
+    // batch against 8,700 on the per-simulation kernel); delayed networks run in blocks of
+    // 32 steps (integrate_delay.cuh: 1,000-node WC, 148 sims: 31,000 cycles per sim-step
+    // and SM against the lane kernel's 66,000), everything else on the per-simulation
+    // kernel.  The lane kernel runs the G tangent, and when
     // CBNM_FP32_KERNEL=lanes or the tuner picks it; CBNM_FP32_KERNEL=simt forces the
     // per-simulation kernel.
     const char *fp32_kernel = std::getenv("CBNM_FP32_KERNEL");
@@ -962,7 +977,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         if (!ok) throw Err(CBNM_ERR_UNSUPPORTED, std::string("integrator variant ") + kVariantName[variant] +
                                                      " does not apply to this run");
     }
-    const bool use_tc = variant == V_DEFAULT ? (!tan_bold && !force_simt && tc_ok)
+    // (CBNM_FP32_KERNEL=lanes leaves networks the 32-wide tiles hold, <= 128 nodes, on the tiles)
+    const bool use_tc = variant == V_DEFAULT ? (!tan_bold && !force_simt && tc_ok && !(force_lanes && n > 128))
                                              : (variant == V_PP || variant == V_PPWS || variant == V_V5);
     bool use_lanes = variant == V_DEFAULT ? (lanes_ok && (tan_bold || (force_lanes && !use_tc)))
                                           : (variant == V_LANES || variant == V_LANES512);
@@ -1055,29 +1071,10 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     ia.do_fic = c.do_fic; ia.max_fic_trials = c.max_fic_trials; ia.I_start = c.I_start; ia.I_end = c.I_end;
     ia.I_dur = c.I_dur; ia.init_delta = c.init_delta;
     ia.bw = g_bw; ia.bw.dt = c.bw_dt; ia.bw.dt_itau = ia.bw.dt * ia.bw.itau;  // core.cpp:291-292
-    {  // C(1/alpha, k) for the FP32 kernel's binomial form of nu^(1/alpha)
-        long double v = 1.0L;
-        ia.bw_binom[0] = 1.0;
-        for (int k = 1; k <= 12; ++k) {
-            v = v * ((long double)ia.bw.ialpha - (k - 1)) / k;
-            ia.bw_binom[k] = (double)v;
-        }
-    }
     ia.K = make_constants(md.id, c.dt);
     for (int i = 0; i < 24; ++i) ia.Kf.all[i] = (float)ia.K.all[i];
-    {  // the two-tile kernel reads these from its parameter space
-        BWFast &f = ia.bwf;
-        f.dt = ia.bw.dt; f.kappa = ia.bw.kappa; f.y = ia.bw.y; f.dt_itau = ia.bw.dt_itau; f.ialpha = ia.bw.ialpha;
-        f.irho = 1.0 / ia.bw.rho; f.log2_omr = std::log2(ia.bw.oneminrho); f.ln_omr = std::log(ia.bw.oneminrho);
-        f.omr = ia.bw.oneminrho;
-        f.V0k1 = ia.bw.V_0 * ia.bw.k1; f.V0k2 = ia.bw.V_0 * ia.bw.k2; f.V0k3 = ia.bw.V_0 * ia.bw.k3;
-        std::copy(ia.bw_binom, ia.bw_binom + 13, f.binom);
-        if (md.id == MODEL_RWW) {
-            const RWW32::K k = RWW32::make(ia.K);
-            static_assert(sizeof(k) <= sizeof(ia.k32), "FP32 constants");
-            std::memcpy(ia.k32, &k, sizeof(k));
-        }
-    }
+    fill_bwf(ia);
+    fill_k32(md.id, ia.K, ia.k32);   // the tensor-core kernels' constants
     ia.sim_begin = 0;
     ia.n_regional = md.n_regional;
     ia.status = d_status;
@@ -1131,7 +1128,14 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         }
         CK(cudaStreamSynchronize(S.st));  // host vectors go out of scope
     }
-    if (!use_tc && !delay_blocks) {
+    // FP64 without delays or numerical FIC, up to 128 nodes: the register-resident forms
+    // (integrate_tile64.cu) unless a coupling form of the per-simulation kernel is forced.
+    // Up to four simulations per SM run one per CTA, more in tiles of eight: at 100 nodes a
+    // step of a tile takes about four times a single simulation's, and N / 8 tiles must
+    // fill the SMs.
+    const bool t64 = !c.fp32 && !has_delay && !num_fic && tile64_supported(md.id, n) && !std::getenv("CBNM_COUPLING");
+    const bool t64_tiles = t64 && N > 4 * sm_count();
+    if (!use_tc && !delay_blocks && !t64) {
         // Sparse coupling for the per-simulation kernels (ELLPACK by target node):
         // used when the densest column of every SC holds at most half the nodes
         // (CBNM_COUPLING=sparse|dense overrides).  Zero weights are skipped and the
@@ -1215,10 +1219,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
                         (variant == V_DEFAULT ? pp_env : (variant == V_PP || variant == V_PPWS));
     // the warp-specialised two-tile form: CBNM_FP32_TC=ws, or the tuned variant
     const bool pp_ws = use_pp && (variant == V_DEFAULT ? (tc_kind && std::string(tc_kind) == "ws") : variant == V_PPWS);
-    if (use_tc) {
-        // tiles of simulations that share one SC
-        const int TN = use_pp ? 32 : fp32_tile_for(n);
-        ia.tile_width = TN;
+    // tiles of TN simulations that share one SC: [n][1 + TN] = SC index, simulation ids (-1 = empty)
+    auto make_tiles = [&](int TN) {
         std::vector<int> sc_of(N);
         if (device_io) {
             if (h_sc_idx.size() != (size_t)N) {
@@ -1241,16 +1243,31 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
             for (; cnt < TN; ++cnt) tiles.push_back(-1);
         }
         ia.n_tiles = (int)(tiles.size() / (TN + 1));
-        if (use_pp) tiles = pair_tiles(tiles, ia.n_tiles, sm_count(), &ia.n_tiles, &ia.pp_grid);
-        ia.pp_ws = pp_ws ? 1 : 0;
+        return tiles;
+    };
+    auto put_tiles = [&](const std::vector<int> &tiles) {
         S.d_tiles.ensure(sizeof(int) * tiles.size());
         CK(cudaMemcpyAsync(S.d_tiles.p, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, S.st));
         ia.tiles = S.d_tiles.as<int>();
-        if (use_pp) ia.bw_scratch = (double *)S.d_bw_scr.ensure(pp_bw_scratch_bytes(n, ia.pp_grid));
         CK(cudaStreamSynchronize(S.st));
+    };
+    if (use_tc) {
+        // Eight-wide tiles up to 16 simulations per SM (or above 128 nodes), 32-wide above
+        // (100 nodes, cycles per step of the whole batch on 148 SMs: integrate_mma.cu's and
+        // integrate_fp32.cu's header comments).
+        const bool wide = !use_pp && N > 16 * sm_count() && tc32_supported(md.id, n);
+        const int TN = use_pp ? 32 : wide ? FP32_TILE_TC : FP32_TILE;
+        std::vector<int> tiles = make_tiles(TN);
+        if (use_pp) tiles = pair_tiles(tiles, ia.n_tiles, sm_count(), &ia.n_tiles, &ia.pp_grid);
+        ia.pp_ws = pp_ws ? 1 : 0;
+        put_tiles(tiles);
+        if (use_pp) ia.bw_scratch = (double *)S.d_bw_scr.ensure(pp_bw_scratch_bytes(n, ia.pp_grid));
         CK(cudaEventRecord(S.ev[1], S.st));
         if (use_pp) CK(launch_integrate_pp(md.id, ia, S.st, &launches));
-        else CK(launch_integrate_fp32(md.id, ia, S.st, &launches));
+        else {
+            CK((wide ? launch_integrate_tc32 : launch_integrate_mma)(md.id, ia, S.st));
+            ++launches;
+        }
     } else if (use_lanes) {
         // groups of 16 simulations sharing SC and delay table (bnm.cu runs one
         // CTA per simulation; here one CTA integrates a group)
@@ -1322,6 +1339,11 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         CK(cudaStreamSynchronize(S.st));
         CK(cudaEventRecord(S.ev[1], S.st));
         CK(launch_integrate_simt32(md.id, ia, S.st));
+        ++launches;
+    } else if (t64) {
+        if (t64_tiles) put_tiles(make_tiles(FP64_TILE));
+        CK(cudaEventRecord(S.ev[1], S.st));
+        CK(launch_integrate_tile64(md.id, ia, S.st));
         ++launches;
     } else {
         CK(launch_integrate_fp64(md.id, ia, S.st));
@@ -1521,6 +1543,7 @@ static AdjArgs adjoint_args(Session &S, AdjPlan &P, const cbnm_run_args *a) {
     ia.bw = g_bw; ia.bw.dt = c.bw_dt; ia.bw.dt_itau = ia.bw.dt * ia.bw.itau;  // core.cpp:291-292
     ia.K = make_constants(MODEL_RWW, c.dt);
     for (int i = 0; i < 24; ++i) ia.Kf.all[i] = (float)ia.K.all[i];
+    fill_bwf(ia);
     A.sct_f32 = S.d_sct_f32.as<float>();
     A.seg_bw = P.seg_bw; A.n_seg = P.n_seg;
     return A;

@@ -253,7 +253,7 @@ struct WC32 {  // wc.cpp:51-80 in FP32
     static constexpr bool PAIR = false;
     static constexpr int NP = 9, NS = 2, NN = 2, NOUT = 2, CV = 0, BV = 0;
     struct K { float dt, sqdt, itE, itI, aE, aI, muE, muI; };
-    __device__ static K make(const ModelK &m) {
+    __host__ __device__ static K make(const ModelK &m) {
         const WCK &w = m.wc;
         return K{(float)w.dt, (float)w.sqrt_dt, (float)w.itau_E, (float)w.itau_I, (float)w.a_E, (float)w.a_I,
                  (float)w.mu_E, (float)w.mu_I};
@@ -279,7 +279,7 @@ struct RWWEx32 {  // rwwex.cpp:48-73 in FP32
     static constexpr bool PAIR = false;
     static constexpr int NP = 4, NS = 1, NN = 1, NOUT = 3, CV = 0, BV = 0;
     struct K { float JN, a, b, d, id, dit, dg, sqdt; };
-    __device__ static K make(const ModelK &m) {
+    __host__ __device__ static K make(const ModelK &m) {
         const RWWExK &w = m.rwwex;
         return K{(float)w.J_N, (float)w.a, (float)w.b, (float)w.d, (float)(1.0 / w.d), (float)w.dt_itau,
                  (float)w.dt_gamma, (float)w.sqrt_dt};
@@ -300,7 +300,7 @@ struct JR32 {  // jr.cpp:80-133 in FP32
     static constexpr bool PAIR = false;
     static constexpr int NP = 7, NS = 8, NN = 1, NOUT = 8, CV = 7, BV = 6;
     struct K { float dt, sqdt, A, B, a, b, v0, numax2, r, mu, cmin, cmax, mid, asq, bsq; };
-    __device__ static K make(const ModelK &m) {
+    __host__ __device__ static K make(const ModelK &m) {
         const JRK &j = m.jr;
         return K{(float)j.dt, (float)j.sqrt_dt, (float)j.A, (float)j.B, (float)j.a, (float)j.b, (float)j.v0,
                  (float)(2.0 * j.nu_max), (float)j.r, (float)j.mu, (float)j.cmin, (float)j.cmax, (float)j.midpoint,
@@ -338,14 +338,15 @@ struct JR32 {  // jr.cpp:80-133 in FP32
 //                coefficients C(a,k) are computed once on the host; error <= 3 ulp)
 //   (1-rho)^(1/f) = (1-rho) exp(ln(1-rho) (1-f)/f), exp by its Taylor series to
 //                y^10/10!, |y| <= 0.06 (first omitted term < 1e-18)
-//   1/x        = float reciprocal refined by two Newton steps (<= 1 ulp)
+//   1/x        = approximate reciprocal (20 bits) refined by two Newton steps (<= 1 ulp)
 // Outside that range the general exp2 / log2 forms and IEEE division are used.
 constexpr int BINOM_TERMS = 12;
 using BW64 = BWFast;
 static_assert(sizeof(BWFast::binom) == sizeof(double) * (BINOM_TERMS + 1), "binomial terms");
 
 __device__ __forceinline__ double rcp_fast(double x) {
-    double r = (double)__frcp_rn((float)x);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     r = r * fma(-x, r, 2.0);
     return r * fma(-x, r, 2.0);
 }
@@ -404,11 +405,60 @@ __device__ __forceinline__ double bold64(double q, double nu, const BW64 &c) {
     return fma(c.V0k3, __dsub_rn(1.0, nu), b);
 }
 
+// The step of N items.  Where all are within the series' range (every haemodynamic
+// state in practice) there is no branch, so the items' chains of dependent FP64
+// operations overlap: with the range tests of bw_step64 inside, two items took 2,700
+// cycles one after the other in the tile kernel.  Same operations, same results.
+template <int N>
+__device__ __forceinline__ void bw_step64_n(double (&x)[N], double (&f)[N], double (&nu)[N], double (&q)[N],
+                                            const double (&z)[N], const BW64 &c) {
+    bool in_range = true;   // a step moves nu by at most dt/tau |f - nu^a|, so the new nu stays below 1/8 too
+#pragma unroll
+    for (int u = 0; u < N; ++u) in_range = in_range && fabs(nu[u] - 1.0) <= 0.12 && fabs(f[u] - 1.0) <= 0.12;
+    if (!(in_range && c.dt_itau <= 0.002)) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) bw_step64(x[u], f[u], nu[u], q[u], z[u], c);
+        return;
+    }
+    double tf[N], inv_f[N], p[N], e[N], y[N], r[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        double t = fma(-c.kappa, x[u], z[u]);
+        t = fma(-c.y, __dsub_rn(f[u], 1.0), t);
+        x[u] = fma(c.dt, t, x[u]);
+        tf[u] = fma(c.dt, x[u], f[u]);
+        inv_f[u] = rcp_fast(f[u]);
+        p[u] = c.binom[BINOM_TERMS];
+        y[u] = c.ln_omr * ((1.0 - f[u]) * inv_f[u]);
+        e[u] = exp_tiny(y[u]);
+    }
+#pragma unroll
+    for (int k = BINOM_TERMS - 1; k >= 0; --k)
+#pragma unroll
+        for (int u = 0; u < N; ++u) p[u] = fma(p[u], nu[u] - 1.0, c.binom[k]);
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        nu[u] = fma(c.dt_itau, __dsub_rn(f[u], p[u]), nu[u]);
+        r[u] = rcp_fast(nu[u]);
+        p[u] = c.binom[BINOM_TERMS];
+    }
+#pragma unroll
+    for (int k = BINOM_TERMS - 1; k >= 0; --k)
+#pragma unroll
+        for (int u = 0; u < N; ++u) p[u] = fma(p[u], nu[u] - 1.0, c.binom[k]);
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const double in = __dmul_rn(__dmul_rn(f[u], __dsub_rn(1.0, c.omr * e[u])), c.irho);
+        const double out = __dmul_rn(__dmul_rn(p[u], q[u]), r[u]);
+        q[u] = fma(c.dt_itau, __dsub_rn(in, out), q[u]);
+        f[u] = tf[u];
+    }
+}
+
 __device__ __forceinline__ void bw_step64x2(double (&x)[2], double (&f)[2], double (&nu)[2], double (&q)[2],
                                             double z0, double z1, const BW64 &c) {
     const double z[2] = {z0, z1};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) bw_step64(x[u], f[u], nu[u], q[u], z[u], c);
+    bw_step64_n<2>(x, f, nu, q, z, c);
 }
 
 // The same step with the multiply-adds left to the compiler.  The two-tile
