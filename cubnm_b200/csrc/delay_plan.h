@@ -13,7 +13,7 @@ constexpr int DELAY_BLOCK = 32;          // integration steps per block of the k
 constexpr int DELAY_SMEM_SM = 227 * 1024;   // shared memory of an SM that CTAs can use, and 1 KB of it per CTA is the system's
 
 struct DelayPlan {
-    int window = 0, tiles = 0, tile_src = 0, bufs = 1, threads = 0, blob_max = 0, buf_bytes = 0, buf_at = 0, noise_steps = 0;
+    int window = 0, tiles = 0, tile_src = 0, bufs = 1, threads = 0, blob_max = 0, buf_bytes = 0, passes = 1, buf_at = 0, noise_at = 0, noise_steps = 0;
     int smem = 0, n_pairs = 0, near_k = 1, far_max = 0;
     std::vector<int> pair, blob_at, near, near_cnt, near_min;
     std::vector<unsigned char> blob;
@@ -36,7 +36,7 @@ inline std::vector<std::pair<int, int>> delay_pairs(DelayPlan &p, int n_sims, co
     return pairs;
 }
 
-// A tile's entry lists, 16-byte aligned: this header, unsigned end[n] (low half: pairs of
+// A tile's entry lists (per pass over the targets), 16-byte aligned: this header, unsigned end[targets] (low half: pairs of
 // far entries up to and with the target's, high half: near entries), then at the byte
 // offsets given: far offsets into the tile's windows of x(t0 - d) (16 bits each, a
 // target's padded to a pair by repeating one with weight 0), their weights, near codes
@@ -54,7 +54,8 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
     p.blob.clear();
     p.blob_at.clear();
     p.blob_max = 0;
-    std::vector<unsigned> end(n);
+    const int nh = (n + p.passes - 1) / p.passes;
+    std::vector<unsigned> end(nh);
     std::vector<uint16_t> off;
     std::vector<int> noff;
     std::vector<R> w, nw;
@@ -62,10 +63,11 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
     for (const auto &pr : pairs) {
         const double *S = sc + (size_t)pr.first * nn;
         const int *d = delay.data() + (size_t)pr.second * nn;
-        for (int t = 0; t < p.tiles; ++t) {
-            const int s0 = t * p.tile_src, s1 = std::min(n, s0 + p.tile_src);
+        for (int pt = 0; pt < p.passes * p.tiles; ++pt) {
+            const int pass = pt / p.tiles, t = pt % p.tiles;
+            const int s0 = t * p.tile_src, s1 = std::min(n, s0 + p.tile_src), h0 = pass * nh, h1 = std::min(n, h0 + nh);
             off.clear(); w.clear(); noff.clear(); nw.clear();
-            for (int j = 0; j < n; ++j) {
+            for (int j = h0; j < h1; ++j) {
                 for (int k = s0; k < s1; ++k) {
                     const double v = S[(size_t)k * n + j];
                     if (v == 0.0) continue;
@@ -83,10 +85,10 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
                     w.push_back(R(0));
                 }
                 if (off.size() / 2 > 0xffff || noff.size() > 0xffff) return false;
-                end[j] = (unsigned)(off.size() / 2) | ((unsigned)noff.size() << 16);
+                end[j - h0] = (unsigned)(off.size() / 2) | ((unsigned)noff.size() << 16);
             }
             TileHead h;
-            h.off_at = (int)up16(sizeof(h) + sizeof(unsigned) * n);
+            h.off_at = (int)up16(sizeof(h) + sizeof(unsigned) * nh);
             h.w_at = (int)up16(h.off_at + sizeof(uint16_t) * off.size());
             h.near_at = (int)up16(h.w_at + sizeof(R) * w.size());
             h.near_w_at = (int)up16(h.near_at + sizeof(int) * noff.size());
@@ -95,7 +97,7 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
             p.blob.resize(at + bytes);
             unsigned char *b = p.blob.data() + at;
             std::memcpy(b, &h, sizeof(h));
-            std::memcpy(b + sizeof(h), end.data(), sizeof(unsigned) * n);
+            std::memcpy(b + sizeof(h), end.data(), sizeof(unsigned) * (h1 - h0));
             if (!off.empty()) {
                 std::memcpy(b + h.off_at, off.data(), sizeof(uint16_t) * off.size());
                 std::memcpy(b + h.w_at, w.data(), sizeof(R) * w.size());
@@ -106,8 +108,8 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
             }
             p.blob_max = std::max(p.blob_max, (int)bytes);
             if (p.blob.size() > max_bytes) return false;
+            if (t == p.tiles - 1) p.blob_at.push_back((int)(p.blob.size() / 16));
         }
-        p.blob_at.push_back((int)(p.blob.size() / 16));
     }
     return true;
 }
@@ -165,20 +167,30 @@ inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int s
     const int least = (n + 31) / 32 * 32;
     const bool f64 = sizeof(R) == 8;
     const int rows = (int)(sizeof(R) * n * (DELAY_BLOCK + 1) + 15) & ~15;
-    p.buf_at = rows;
     const double nnz_node = (double)nnz / n;
-    const double per_src = (double)p.window * sizeof(R) + (nnz_node + n * 0.3) * (2 + sizeof(R));   // window and entries
     const int thr_sm = f64 ? 512 : 1024;   // by registers, see min_ctas
+    const int step_bytes = (int)sizeof(R) * n * n_noise;   // noise of a step
     for (int c = std::min({8, (n_sims + sms - 1) / sms, std::max(1, thr_sm / least)}); c >= 1; --c) {
-        const double space = DELAY_SMEM_SM / c - 1024 - p.buf_at - 4.0 * n - 256;
-        auto fit = [&](int bufs) { return std::min<int>({n, 65535 / p.window, (int)((space - (bufs - 1) * 4.0 * n) / bufs / per_src)}); };
-        p.bufs = 1;
+        const int most_smem = DELAY_SMEM_SM / c - 1024;
+        auto fit = [&](int bufs) {   // sources whose windows and entries, with row ends and padding, fill a buffer
+            const double fixed = (double)n / p.passes * (4 + 0.6 * (2 + sizeof(R))) + 512;
+            const double src = (double)p.window * sizeof(R) + nnz_node / p.passes * 1.1 * (2 + sizeof(R));
+            return std::min<int>({n, 65535 / p.window, (int)(((most_smem - p.buf_at) / bufs - fixed) / src)});
+        };
+        p.bufs = p.passes = 1;
+        p.buf_at = p.noise_at = rows;
         p.tile_src = fit(1);
         if (p.tile_src < n && c == 1 && nnz_node * fit(2) / n >= 12.0) {   // alone on its SM: load during the gather
             p.bufs = 2;
             p.tile_src = fit(2);
         }
         if (c > 1 && p.tile_src < n && nnz_node * p.tile_src / n < 3.0) continue;
+        if (!f64 && n > 512 && c == 1 && p.tile_src < n && nnz_node * p.tile_src / n < 6.0 &&
+             most_smem - rows >= 4 * (step_bytes + (int)sizeof(R) * n)) {
+            p.passes = 2;                          // half the sums, larger tiles; then at least 4 steps of noise and sums
+            p.buf_at = ((int)sizeof(R) * ((n + 1) / 2) * (DELAY_BLOCK + 1) + 15) & ~15;
+            p.tile_src = fit(1);
+        }
         if (p.tile_src < std::min(n, 4)) continue;
         const int most = c == 1 ? (f64 ? 512 : n <= 256 ? 512 : 1024) : std::min(f64 ? 256 : 512, thr_sm / c / 32 * 32);
         p.threads = std::max(least, most);
@@ -186,8 +198,9 @@ inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int s
             if (!delay_blobs<R>(p, n, sc, delay, pairs, max_bytes)) return false;
             p.buf_bytes = ((p.blob_max + p.tile_src * p.window * (int)sizeof(R)) + 15) & ~15;
             p.smem = p.buf_at + p.bufs * p.buf_bytes;
-            if (p.smem <= DELAY_SMEM_SM / c - 1024) {
-                p.noise_steps = std::min(DELAY_BLOCK, p.bufs * p.buf_bytes / (int)(sizeof(R) * n * n_noise));
+            if (p.smem <= most_smem) {
+                if (p.passes == 2) p.smem = most_smem & ~15;
+                p.noise_steps = std::min(DELAY_BLOCK, (p.smem - p.noise_at - 16) / (step_bytes + (p.passes == 2 ? (int)sizeof(R) * ((n + 3) & ~3) : 0)));
                 return p.noise_steps > 0;
             }
             p.tile_src = (int)(p.tile_src * 0.93);

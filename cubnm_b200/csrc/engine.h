@@ -148,10 +148,12 @@ struct IntegrateArgs {
     int db_bufs;                 // tile buffers in shared memory (2: the next tile loads during this one)
     int db_blob_max;             // bytes reserved for a tile's entry lists in a buffer
     int db_buf_bytes;            // bytes of a buffer (entry lists, then windows)
-    int db_buf_at;               // shared-memory offset of the buffers
+    int db_passes;               // 2: half of the targets' sums at a time (FP32, large networks)
+    int db_buf_at, db_noise_at;  // shared-memory offsets of the buffers and, during the steps, of the noise
+    void *db_sums;               // two passes: [CTA][32][nodes padded to 4] sums of a block
     int db_noise_steps;          // steps of noise the buffers hold (at most 32)
     const int *db_pair;          // [n_sims] pair of each simulation
-    const int *db_blob_at;       // [n_pairs][db_tiles + 1] start of each tile's lists, in 16 bytes
+    const int *db_blob_at;       // [n_pairs][db_passes][db_tiles + 1] start of each tile's lists, in 16 bytes
     const void *db_blob;         // entry lists (delay_plan.h)
     int db_near_k;               // entries per near list (the longest of any pair)
     const int *db_near;          // [n_pairs][db_near_k][nodes] near: source * 32 + delay (0: padding)

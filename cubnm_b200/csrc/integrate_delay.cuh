@@ -19,6 +19,9 @@
 //     barrier (of the warps that hold nodes) is due every min(near d) steps; with no
 //     near pair there is none.  The noise of the steps is copied to shared memory
 //     beforehand, into the tile buffers, which are free now.
+//     (Networks whose 32 sums per node leave little shared memory for tiles gather them in
+//     two passes over the targets, the sums parked in global memory and brought back in
+//     chunks with the noise: at 1,000 nodes tiles of 73 sources instead of 25.)
 //  3. the block's 32 values per node go to the ring buffer, one line per node.
 //
 // What bounds it: step 1 is shared-memory bandwidth (one wavefront per entry and 32
@@ -46,6 +49,7 @@ struct Arr;
 template <>
 struct Arr<float> {
     __device__ static float *hist(const IntegrateArgs &a) { return a.hist_f32; }
+    __device__ static float *sums(const IntegrateArgs &a) { return static_cast<float *>(a.db_sums); }
     __device__ static const float *near_w(const IntegrateArgs &a) { return a.db_near_w32; }
     __device__ static const ModelKf &consts(const IntegrateArgs &a) { return a.Kf; }
     __device__ static void pair(const float *w, unsigned p, float &w0, float &w1) {
@@ -57,6 +61,7 @@ struct Arr<float> {
 template <>
 struct Arr<double> {
     __device__ static double *hist(const IntegrateArgs &a) { return a.hist; }
+    __device__ static double *sums(const IntegrateArgs &a) { return static_cast<double *>(a.db_sums); }
     __device__ static const double *near_w(const IntegrateArgs &a) { return a.db_near_w64; }
     __device__ static const ModelK &consts(const IntegrateArgs &a) { return a.K; }
     __device__ static void pair(const double *w, unsigned p, double &w0, double &w1) {
@@ -81,10 +86,10 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 // Copies tile `t` to buf: the entry lists (one 16-byte-aligned blob), then the window
 // of each source, the ring rotated so that it ends at t0.
 template <class R>
-__device__ __forceinline__ void stage_tile(const IntegrateArgs &a, int pair, int t, const R *hist, unsigned char *buf,
-                                           int t0m) {
+__device__ __forceinline__ void stage_tile(const IntegrateArgs &a, int pair, int pass, int t, const R *hist,
+                                           unsigned char *buf, int t0m) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int *at = a.db_blob_at + (size_t)pair * (a.db_tiles + 1) + t;
+    const int *at = a.db_blob_at + ((size_t)pair * a.db_passes + pass) * (a.db_tiles + 1) + t;
     const int b0 = __ldg(at), b1 = __ldg(at + 1);   // in units of 16 bytes
     const int4 *src = reinterpret_cast<const int4 *>(a.db_blob) + b0;
     for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) cp16(buf + 16 * (size_t)i, src + i);
@@ -105,33 +110,42 @@ __device__ __forceinline__ void stage_tile(const IntegrateArgs &a, int pair, int
 // row (time shuffle, inner step), column = the repeat's node shuffle.  sh_ts is
 // [repeats][noise_bw_it], one run of Balloon-Windkessel steps.
 template <int NN, class R>
-__device__ __noinline__ void stage_noise(const IntegrateArgs &a, const R *noise, int t, int steps, unsigned char *buf) {
+__device__ __noinline__ void stage_noise(const IntegrateArgs &a, const R *noise, int t, int steps, R *buf) {
     const int n = a.nodes, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int q = warp; q < steps; q += nwarps) {
-        const int bw = (t + q) / a.inner_it, inner = (t + q) - bw * a.inner_it;
-        const R *src = noise + ((long long)__ldg(a.sh_ts + bw) * a.inner_it + inner) * n * NN;
-        const int *shn = a.sh_nodes + (size_t)(bw / a.noise_bw_it) * n;
-        R *dst = reinterpret_cast<R *>(buf) + (size_t)q * n * NN;
-        for (int k = lane; k < n; k += 32) cp_small<NN * (int)sizeof(R)>(dst + k * NN, src + (size_t)__ldg(shn + k) * NN);
+    const int chunks = (n + 31) >> 5;   // (step, 32 nodes) pairs over the warps
+    int q = warp / chunks, c = warp - q * chunks;
+    const int dq = nwarps / chunks, dc = nwarps - dq * chunks;
+#pragma unroll 2
+    for (; q < steps;) {
+        const int k = c * 32 + lane;
+        if (k < n) {
+            const int bw = (t + q) / a.inner_it, inner = (t + q) - bw * a.inner_it;
+            const int shk = __ldg(a.sh_nodes + (size_t)(bw / a.noise_bw_it) * n + k);
+            const R *src = noise + ((long long)__ldg(a.sh_ts + bw) * a.inner_it + inner) * n * NN;
+            cp_small<NN * (int)sizeof(R)>(buf + ((size_t)q * n + k) * NN, src + (size_t)shk * NN);
+        }
+        q += dq;
+        c += dc;
+        if (c >= chunks) { c -= chunks; ++q; }
     }
 }
 
-// Step 1 of a block.  Out of line, so that the node state's registers are saved once
-// per block instead of limiting this loop.
+// Step 1 of a block: the sums of targets [h0, h1) into row[target - h0][lane].  Out of line,
+// so that the node state's registers are saved once per block instead of limiting this loop.
 template <class R>
-__device__ __noinline__ void gather_block(const IntegrateArgs &a, int pair, const R *hist, R *row, unsigned char *bufs,
-                                          int t0m) {
+__device__ __noinline__ void gather_block(const IntegrateArgs &a, int pair, int pass, int h0, int h1, const R *hist,
+                                          R *row, unsigned char *bufs, int t0m) {
     using A = Arr<R>;
-    const int n = a.nodes, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int k0 = (int)((long long)n * warp / nwarps), k1 = (int)((long long)n * (warp + 1) / nwarps);
+    const int nh = h1 - h0, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int k0 = (int)((long long)nh * warp / nwarps), k1 = (int)((long long)nh * (warp + 1) / nwarps);
     const int tiles = a.db_tiles;
     const bool two = a.db_bufs == 2;
-    stage_tile<R>(a, pair, 0, hist, bufs, t0m);
+    stage_tile<R>(a, pair, pass, 0, hist, bufs, t0m);
     cp_commit();
     for (int t = 0; t < tiles; ++t) {
         unsigned char *buf = bufs + (two ? (t & 1) * (size_t)a.db_buf_bytes : 0);
         if (two && t + 1 < tiles) {
-            stage_tile<R>(a, pair, t + 1, hist, bufs + ((t + 1) & 1) * (size_t)a.db_buf_bytes, t0m);
+            stage_tile<R>(a, pair, pass, t + 1, hist, bufs + ((t + 1) & 1) * (size_t)a.db_buf_bytes, t0m);
             cp_commit();
             cp_wait<1>();
         } else {
@@ -166,7 +180,7 @@ __device__ __noinline__ void gather_block(const IntegrateArgs &a, int pair, cons
         }
         __syncthreads();   // the buffer is free; after the last tile the sums are complete
         if (!two && t + 1 < tiles) {
-            stage_tile<R>(a, pair, t + 1, hist, bufs, t0m);
+            stage_tile<R>(a, pair, pass, t + 1, hist, bufs, t0m);
             cp_commit();
         }
     }
@@ -201,13 +215,20 @@ __global__ void __launch_bounds__(MAXT, min_ctas<R, MAXT>()) k_integrate_delay(c
     static_assert(!M::OSC, "the phase model's coupling depends on the target's current phase");
     using A = Arr<R>;
     using P = typename M::P;
+    constexpr bool TWO = sizeof(R) == 4 && MAXT == 1024;   // two passes over the targets are possible
+    const bool two = TWO && a.db_passes == 2;
     const int n = a.nodes;
     const int j = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const bool act = j < n;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *row = reinterpret_cast<R *>(smem_raw);   // [n][DROW]
     unsigned char *bufs = smem_raw + a.db_buf_at;
-    const R *nz = reinterpret_cast<const R *>(bufs) + (size_t)j * M::NN;   // noise of a chunk of steps [step][n][NN]
+    // during the steps: noise of a chunk of them [step][n][NN], with two passes then their sums [step][n]
+    R *const nzb = reinterpret_cast<R *>(smem_raw + a.db_noise_at);
+    const R *nz = nzb + (size_t)j * M::NN;
+    const int ns = (n + 3) & ~3;   // row of sums
+    R *const sum_s = nzb + (((size_t)a.db_noise_steps * n * M::NN + 3) & ~(size_t)3);
+    R *const sums = two ? A::sums(a) + (size_t)blockIdx.x * DB * ns : nullptr;
     const int node_threads = (n + 31) & ~31;
     __shared__ int s_trial, s_adjust, s_failed;
     const int W = a.db_window;
@@ -263,7 +284,18 @@ __global__ void __launch_bounds__(MAXT, min_ctas<R, MAXT>()) k_integrate_delay(c
                 __syncthreads();
             }
             // ---- 1. gather, lane = step of the block
-            gather_block<R>(a, pair, hist, row, bufs, t0m);
+            if (!two) {
+                gather_block<R>(a, pair, 0, 0, n, hist, row, bufs, t0m);
+            } else {   // half of the targets at a time; their sums wait in global memory, [step][node]
+                const int nh = (n + 1) / 2;
+                for (int h = 0; h < 2; ++h) {
+                    const int h0 = h * nh, h1 = min(n, h0 + nh);
+                    gather_block<R>(a, pair, h, h0, h1, hist, row, bufs, t0m);
+                    for (int b = warp; b < DB; b += nwarps)
+                        for (int k = h0 + lane; k < h1; k += 32) sums[(size_t)b * ns + k] = row[(k - h0) * DROW + b];
+                    __syncthreads();
+                }
+            }
             // ---- 2. the block's steps, thread = node, in chunks of the noise that the buffers hold
             const int nb = min(DB, total - t0);
             bool restart = false;
@@ -271,7 +303,11 @@ __global__ void __launch_bounds__(MAXT, min_ctas<R, MAXT>()) k_integrate_delay(c
             for (int b = 0; b < nb;) {
                 if (b % a.db_noise_steps == 0) {
                     if (b) __syncthreads();   // the previous chunk is used
-                    stage_noise<M::NN, R>(a, noise, t0 + b, min(a.db_noise_steps, nb - b), bufs);
+                    const int cnt = min(a.db_noise_steps, nb - b);
+                    stage_noise<M::NN, R>(a, noise, t0 + b, cnt, nzb);
+                    if (two)
+                        for (int i = threadIdx.x * 4; i < cnt * ns; i += blockDim.x * 4)
+                            cp16(sum_s + i, sums + (size_t)b * ns + i);
                     cp_commit();
                     cp_wait<0>();
                     __syncthreads();
@@ -286,7 +322,7 @@ __global__ void __launch_bounds__(MAXT, min_ctas<R, MAXT>()) k_integrate_delay(c
                             next_sync += sync_every;
                         }
                         if (!act) continue;
-                        R in = row[j * DROW + b];
+                        R in = two ? sum_s[(b - chunk) * ns + j] : row[j * DROW + b];
                         const R *z = nz + (size_t)(b - chunk) * n * M::NN;
                         const R n0 = z[0], n1 = M::NN > 1 ? z[1] : R(0);
                         if (near_n) {  // d = 0: the padding of shorter lists
@@ -424,6 +460,8 @@ cudaError_t occupancy(const DelayLaunch &c, int *occ) {
 
 template <class M, class R>
 cudaError_t config_model(const IntegrateArgs &a, int sms, DelayLaunch *c) {
+    // the two-pass form is compiled for the FP32 kernel of more than 512 threads only
+    if (a.db_passes != 1 && (sizeof(R) != 4 || c->threads <= 512)) return cudaErrorInvalidValue;
     int occ = 0;
     const cudaError_t e = c->threads <= 256   ? occupancy<M, R, 256>(*c, &occ)
                           : c->threads <= 512 ? occupancy<M, R, 512>(*c, &occ)

@@ -344,7 +344,7 @@ struct Session {
     DBuf d_bold, d_states, d_gbools, d_gints, d_fc, d_fcd, d_wfc, d_pairs_i, d_pairs_j, d_wstart, d_wend, d_status;
     DBuf d_tiles, d_sct_f32, d_ell_pk, d_bw_scr, d_ln_groups, d_ln_params, d_ln_hist, d_ln_bw;
     DBuf fl_ec, fl_q, fl_win, fl_scr;  // fit loss
-    DBuf d_db_pair, d_db_at, d_db_blob, d_db_near, d_db_near_w, d_db_near_n;  // delay kernel lists
+    DBuf d_db_pair, d_db_at, d_db_blob, d_db_sums, d_db_near, d_db_near_w, d_db_near_n;  // delay kernel lists
     DBuf d_pidx, d_wstat;              // tensor-core FC: pair index of (i, j); window-FC statistics
     // gof
     DBuf g_simfc, g_empfc, g_simfcd, g_empfcd, g_out;
@@ -400,7 +400,7 @@ static void close_session(Session *&p) {
                         &S.d_hist, &S.d_hist_f32, &S.d_bold, &S.d_states, &S.d_gbools, &S.d_gints, &S.d_fc,
                         &S.d_fcd, &S.d_wfc, &S.d_pairs_i, &S.d_pairs_j, &S.d_wstart, &S.d_wend, &S.d_status, &S.d_tiles,
                         &S.d_sct_f32, &S.d_ell_pk, &S.d_bw_scr, &S.d_ln_groups, &S.d_ln_params, &S.d_ln_hist, &S.d_ln_bw, &S.fl_ec, &S.fl_q, &S.fl_win, &S.fl_scr, &S.d_pidx, &S.d_wstat,
-                        &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
+                        &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_sums, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
                         &S.g_simfc, &S.g_empfc, &S.g_simfcd, &S.g_empfcd, &S.g_out})
             b->release();
         for (auto &ev : S.ev) cudaEventDestroy(ev);
@@ -1110,7 +1110,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         if (c.fp32) up(S.d_db_near_w, near_w32.data(), sizeof(float) * near_w32.size());
         else up(S.d_db_near_w, plan.near_w.data(), sizeof(double) * plan.near_w.size());
         ia.db_window = plan.window; ia.db_tiles = plan.tiles; ia.db_tile_src = plan.tile_src; ia.db_bufs = plan.bufs;
-        ia.db_blob_max = plan.blob_max; ia.db_buf_bytes = plan.buf_bytes; ia.db_buf_at = plan.buf_at;
+        ia.db_blob_max = plan.blob_max; ia.db_buf_bytes = plan.buf_bytes; ia.db_buf_at = plan.buf_at; ia.db_noise_at = plan.noise_at; ia.db_passes = plan.passes;
         ia.db_noise_steps = plan.noise_steps;
         ia.db_pair = S.d_db_pair.as<int>(); ia.db_blob_at = S.d_db_at.as<int>(); ia.db_blob = S.d_db_blob.p;
         ia.db_near_k = plan.near_k; ia.db_near = S.d_db_near.as<int>();
@@ -1119,6 +1119,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         dl.smem = plan.smem;
         CK((c.fp32 ? delay_config32 : delay_config64)(md.id, ia, sm_count(), &dl));
         const size_t slots = (size_t)n * plan.window * dl.grid;
+        if (plan.passes == 2)
+            ia.db_sums = S.d_db_sums.ensure((c.fp32 ? sizeof(float) : sizeof(double)) * (size_t)dl.grid * DELAY_BLOCK * ((n + 3) & ~3));
         if (c.fp32) {
             ia.db_near_w32 = S.d_db_near_w.as<float>();
             ia.hist_f32 = (float *)S.d_hist_f32.ensure(sizeof(float) * slots);

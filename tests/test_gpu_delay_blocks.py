@@ -88,3 +88,15 @@ def test_pairs_and_more_simulations_than_ctas():
     ref = oracle.run_simulations(*_copy(b))
     for k in ("sim_bold", "sim_fc_trils"):
         np.testing.assert_allclose(whole[k][pick], ref[k], rtol=1e-8, atol=1e-12, err_msg=k)
+
+
+def test_two_passes_over_the_targets():
+    """Above 512 nodes in FP32 with few entries per tile the sums are formed for half the
+    targets at a time (an odd node count, near pairs, 331 ms = no whole number of blocks)."""
+    nodes = 701
+    dist = _uniform(nodes, 6.0, 190.0)
+    a = _args("rWW", nodes, 3, dist, 6.0, 331, density=0.08)
+    o64 = core.run_simulations(*_copy(a))
+    o32 = core.run_simulations(*_copy(_args("rWW", nodes, 3, dist, 6.0, 331, density=0.08, precision="fp32")))
+    np.testing.assert_allclose(o32["_sim_states"], o64["_sim_states"], rtol=1e-4, atol=1e-5)
+    assert np.abs(o32["sim_bold"] - o64["sim_bold"]).max() < 1e-4
