@@ -12,6 +12,7 @@
 #include <cstdint>
 #include "engine.h"
 #include "models.cuh"
+#include "tc_common.cuh"
 
 namespace cbnm {
 
@@ -50,22 +51,33 @@ struct SimArrays<float> {
 };
 
 // FP32 coupling input of node j, sum_k SC[k][j] x[k] (x in shared memory, 16-byte
-// aligned): four independent partial sums over k = 0,1,2,3 mod 4 (float4 reads
-// of x), so the FMA chain is a quarter as long; combined as (s0 + s1) + (s2 + s3).
-// The FP64 path keeps the reference's sequential order instead.
+// aligned): sixteen partial sums over k mod 16 (float4 reads of x), combined in the
+// tree of the adjoint kernels' lane butterfly (adjoint.cu), so that both give the same
+// bits.  The FP64 path keeps the reference's sequential order instead.
 __device__ __forceinline__ float coupling_f32(const float *__restrict__ SC, const float *x, int n, int j) {
-    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+    float p[16];
+#pragma unroll
+    for (int l = 0; l < 16; ++l) p[l] = 0.0f;
     const float4 *x4 = reinterpret_cast<const float4 *>(x);
     int k = 0;
-    for (; k + 3 < n; k += 4) {
-        const float4 v = x4[k >> 2];
-        s0 += __ldg(&SC[(size_t)k * n + j]) * v.x;
-        s1 += __ldg(&SC[(size_t)(k + 1) * n + j]) * v.y;
-        s2 += __ldg(&SC[(size_t)(k + 2) * n + j]) * v.z;
-        s3 += __ldg(&SC[(size_t)(k + 3) * n + j]) * v.w;
+    for (; k + 15 < n; k += 16) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const float4 v = x4[(k >> 2) + h];
+            p[4 * h] = fmaf(__ldg(&SC[(size_t)(k + 4 * h) * n + j]), v.x, p[4 * h]);
+            p[4 * h + 1] = fmaf(__ldg(&SC[(size_t)(k + 4 * h + 1) * n + j]), v.y, p[4 * h + 1]);
+            p[4 * h + 2] = fmaf(__ldg(&SC[(size_t)(k + 4 * h + 2) * n + j]), v.z, p[4 * h + 2]);
+            p[4 * h + 3] = fmaf(__ldg(&SC[(size_t)(k + 4 * h + 3) * n + j]), v.w, p[4 * h + 3]);
+        }
     }
-    for (; k < n; ++k) s0 += __ldg(&SC[(size_t)k * n + j]) * x[k];
-    return (s0 + s1) + (s2 + s3);
+#pragma unroll
+    for (int l = 0; l < 16; ++l)
+        if (k + l < n) p[l] = fmaf(__ldg(&SC[(size_t)(k + l) * n + j]), x[k + l], p[l]);
+#pragma unroll
+    for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+        for (int l = 0; l < h; ++l) p[l] = p[l] + p[l + h];
+    return p[0];
 }
 
 // MAXT = the block size bound: 1024 (at most 64 registers a thread), or 512 (up
@@ -193,7 +205,10 @@ __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
             }
             if (DELAY) buff = (buff + D - 1) % D;
         }
-        if (act) bw_step(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bw);
+        if (act) {
+            if constexpr (sizeof(R) == 4) bw_step64(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bwf);
+            else bw_step(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bw);
+        }
         if ((bw_i + 1) % a.bold_tr_iters == 0) {  // bnm.cpp:316-335
             // the truncated iteration counts (bw_it, bold_tr_iters) can give one more
             // sample than bold_len for some TR / bw_dt; that sample has no slot
