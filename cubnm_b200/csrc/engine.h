@@ -31,11 +31,15 @@ struct BWConst {
     double ialpha, itau, oneminrho, dt_itau, V_0_k1, V_0_k2, V_0_k3;
 };
 
+// Extents of the table behind BWFast::tab (tc_common.cuh): 17 pairs and 20 values.
+constexpr int BW_NU = 17, BW_NU0 = 8, BW_EXP = 20, BW_EXP0 = 16;
+
 // Balloon-Windkessel constants in the form the FP32 tensor-core kernels use (FP64
 // step with series for the powers, tc_common.cuh): filled on the host.
 struct BWFast {
     double dt, kappa, y, dt_itau, ialpha, irho, log2_omr, ln_omr, omr, V0k1, V0k2, V0k3;
     double binom[13];            // C(1/alpha, k), k = 0..12
+    const double *tab;           // device: {c^-1, c^(1/alpha)} for c = 1.25^(i - BW_NU0), then e^((i - BW_EXP0) / 8)
 };
 
 // Model constants, computed on the host exactly as the reference's

@@ -78,8 +78,9 @@ static BWConst bw_defaults(double dt_s) {  // bw.cpp:4-22
 static BWConst g_bw = bw_defaults(0.001);
 static std::string g_err;
 
-// The Balloon-Windkessel constants of the series form, from ia.bw.
-static void fill_bwf(IntegrateArgs &ia) {
+// The Balloon-Windkessel constants of the series form, from ia.bw; `tab` the session's table.
+static void fill_bwf(IntegrateArgs &ia, const double *tab) {
+    ia.bwf.tab = tab;
     BWFast &f = ia.bwf;
     f.dt = ia.bw.dt; f.kappa = ia.bw.kappa; f.y = ia.bw.y; f.dt_itau = ia.bw.dt_itau; f.ialpha = ia.bw.ialpha;
     f.irho = 1.0 / ia.bw.rho; f.log2_omr = std::log2(ia.bw.oneminrho); f.ln_omr = std::log(ia.bw.oneminrho);
@@ -326,6 +327,7 @@ struct DBuf {
 };
 
 struct Session {
+    DBuf d_bw_tab;               // table of the Balloon-Windkessel powers (bw_table)
     bool ready = false;
     int dev = -1;                // the device the stream, events and buffers belong to
     cudaStream_t st = nullptr;
@@ -387,6 +389,23 @@ static Session &session() {
     return *g_sess;
 }
 
+// The session's table for BWFast::tab, uploaded on first use (1 / alpha is a constant of the model).
+static const double *bw_table(Session &S, double ialpha) {
+    if (!S.d_bw_tab.p) {
+        std::vector<double> t(2 * BW_NU + BW_EXP);
+        for (int i = 0; i < BW_NU; ++i) {
+            const double inv = (double)std::pow(1.25L, (long double)(BW_NU0 - i));
+            t[2 * i] = inv;
+            t[2 * i + 1] = (double)std::pow((long double)inv, -(long double)ialpha);   // the centre is 1 / inv
+        }
+        for (int i = 0; i < BW_EXP; ++i) t[2 * BW_NU + i] = (double)std::exp((long double)(i - BW_EXP0) / 8.0L);
+        S.d_bw_tab.ensure(sizeof(double) * t.size());
+        CK(cudaMemcpyAsync(S.d_bw_tab.p, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice, S.st));
+        CK(cudaStreamSynchronize(S.st));
+    }
+    return S.d_bw_tab.as<double>();
+}
+
 static void close_session(Session *&p) {
     if (!p) return;
     Session &S = *p;
@@ -400,7 +419,7 @@ static void close_session(Session *&p) {
                         &S.d_hist, &S.d_hist_f32, &S.d_bold, &S.d_states, &S.d_gbools, &S.d_gints, &S.d_fc,
                         &S.d_fcd, &S.d_wfc, &S.d_pairs_i, &S.d_pairs_j, &S.d_wstart, &S.d_wend, &S.d_status, &S.d_tiles,
                         &S.d_sct_f32, &S.d_ell_pk, &S.d_bw_scr, &S.d_ln_groups, &S.d_ln_params, &S.d_ln_hist, &S.d_ln_bw, &S.fl_ec, &S.fl_q, &S.fl_win, &S.fl_scr, &S.d_pidx, &S.d_wstat,
-                        &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_sums, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
+                        &S.d_bw_tab, &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_sums, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
                         &S.g_simfc, &S.g_empfc, &S.g_simfcd, &S.g_empfcd, &S.g_out})
             b->release();
         for (auto &ev : S.ev) cudaEventDestroy(ev);
@@ -1073,7 +1092,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     ia.bw = g_bw; ia.bw.dt = c.bw_dt; ia.bw.dt_itau = ia.bw.dt * ia.bw.itau;  // core.cpp:291-292
     ia.K = make_constants(md.id, c.dt);
     for (int i = 0; i < 24; ++i) ia.Kf.all[i] = (float)ia.K.all[i];
-    fill_bwf(ia);
+    fill_bwf(ia, bw_table(S, ia.bw.ialpha));
     fill_k32(md.id, ia.K, ia.k32);   // the tensor-core kernels' constants
     ia.sim_begin = 0;
     ia.n_regional = md.n_regional;
@@ -1545,7 +1564,7 @@ static AdjArgs adjoint_args(Session &S, AdjPlan &P, const cbnm_run_args *a) {
     ia.bw = g_bw; ia.bw.dt = c.bw_dt; ia.bw.dt_itau = ia.bw.dt * ia.bw.itau;  // core.cpp:291-292
     ia.K = make_constants(MODEL_RWW, c.dt);
     for (int i = 0; i < 24; ++i) ia.Kf.all[i] = (float)ia.K.all[i];
-    fill_bwf(ia);
+    fill_bwf(ia, bw_table(S, ia.bw.ialpha));
     A.sct_f32 = S.d_sct_f32.as<float>();
     A.seg_bw = P.seg_bw; A.n_seg = P.n_seg;
     return A;

@@ -332,14 +332,18 @@ struct JR32 {  // jr.cpp:80-133 in FP32
 };
 
 // Balloon-Windkessel step in FP64 (bw.cu:4-15).
-// The powers nu^(1/alpha) and (1-rho)^(1/f) and two divisions dominate its
-// cost.  In the range the haemodynamic state lives in (|nu-1|, |f-1| <= 1/8):
-//   nu^a       = sum_{k<=12} C(a,k) d^k, d = nu - 1 (binomial series; the
-//                coefficients C(a,k) are computed once on the host; error <= 3 ulp)
-//   (1-rho)^(1/f) = (1-rho) exp(ln(1-rho) (1-f)/f), exp by its Taylor series to
-//                y^10/10!, |y| <= 0.06 (first omitted term < 1e-18)
+// The powers nu^(1/alpha) and (1-rho)^(1/f) and two divisions dominate its cost:
+//   nu^a       = c^a (nu/c)^a, c the nearest power of 1.25, (nu/c)^a = sum_{k<=12} C(a,k) d^k,
+//                d = nu/c - 1, |d| <= 0.118 (binomial series; error <= 3 ulp)
+//   (1-rho)^(1/f) = (1-rho) exp(t), t = ln(1-rho) (1-f)/f, exp(t) = e^(i/8) exp(t - i/8), the
+//                last by its Taylor series to y^10/10!, |y| <= 1/16 (first omitted term < 1e-18)
 //   1/x        = approximate reciprocal (20 bits) refined by two Newton steps (<= 1 ulp)
-// Outside that range the general exp2 / log2 forms and IEEE division are used.
+// c^-1, c^a and e^(i/8) come from a small table (filled on the host) that covers
+// nu in [0.15, 6.6] and f > 0.17; outside it the general exp2 / log2 forms and IEEE
+// division are used.  Near rest (c = 1, i = 0) the factors are 1.  A series around 1
+// alone covers |nu - 1|, |f - 1| <= 1/8, which simulations with strong activity leave
+// after a few seconds: the general form in their warps took 900 of 2,800 cycles a step in
+// the eight-wide FP32 tiles (512 simulations, 8 s).
 constexpr int BINOM_TERMS = 12;
 using BW64 = BWFast;
 static_assert(sizeof(BWFast::binom) == sizeof(double) * (BINOM_TERMS + 1), "binomial terms");
@@ -365,19 +369,31 @@ __device__ __forceinline__ double exp_tiny(double y) {  // sum_{k<=10} y^k / k!
     return fma(p, y, 1.0);
 }
 
+// Table index of nu's and of t's centre; in range when the result is in [0, BW_NU) / [0, BW_EXP).
+__device__ __forceinline__ int nu_index(double nu) {
+    const int i = __float2int_rn(__log2f((float)nu) * 3.10628372f) + BW_NU0;   // log_1.25
+    return nu > 0.0 ? i : -1;   // also for a NaN
+}
+__device__ __forceinline__ int exp_index(double t) { return __double2int_rn(t * 8.0) + BW_EXP0; }
+
 __device__ __forceinline__ double pow_nu(double nu, const BW64 &c) {  // nu^(1/alpha)
-    const double d = nu - 1.0;
-    if (fabs(d) <= 0.125) {
+    const int i = nu_index(nu);
+    if ((unsigned)i < (unsigned)BW_NU) {
+        const double2 t = __ldg(reinterpret_cast<const double2 *>(c.tab) + i);
+        const double d = fma(nu, t.x, -1.0);
         double p = c.binom[BINOM_TERMS];
 #pragma unroll
         for (int k = BINOM_TERMS - 1; k >= 0; --k) p = fma(p, d, c.binom[k]);
-        return p;
+        return __dmul_rn(t.y, p);
     }
     return exp2(c.ialpha * log2(nu));
 }
 
 __device__ __forceinline__ double pow_omr(double f, double inv_f, const BW64 &c) {  // (1-rho)^(1/f)
-    if (fabs(f - 1.0) <= 0.125) return c.omr * exp_tiny(c.ln_omr * ((1.0 - f) * inv_f));
+    const double t = __dmul_rn(c.ln_omr, __dmul_rn(__dsub_rn(1.0, f), inv_f));
+    const int i = exp_index(t);
+    if ((unsigned)i < (unsigned)BW_EXP)
+        return __dmul_rn(c.omr, __dmul_rn(__ldg(c.tab + 2 * BW_NU + i), exp_tiny(fma((double)(BW_EXP0 - i), 0.125, t))));
     return exp2(c.log2_omr / f);
 }
 
@@ -405,51 +421,60 @@ __device__ __forceinline__ double bold64(double q, double nu, const BW64 &c) {
     return fma(c.V0k3, __dsub_rn(1.0, nu), b);
 }
 
-// The step of N items.  Where all are within the series' range (every haemodynamic
-// state in practice) there is no branch, so the items' chains of dependent FP64
-// operations overlap: with the range tests of bw_step64 inside, two items took 2,700
-// cycles one after the other in the tile kernel.  Same operations, same results.
+// The step of N items.  Where all are within the table there is no branch, so the items'
+// chains of dependent FP64 operations overlap: with the range tests of bw_step64 inside,
+// two items took 2,700 cycles one after the other in the tile kernel.  The same
+// operations, but the new nu is expanded around the old one's centre, so results differ
+// from bw_step64 in the last bits at a step where nu passes between centres.
 template <int N>
 __device__ __forceinline__ void bw_step64_n(double (&x)[N], double (&f)[N], double (&nu)[N], double (&q)[N],
                                             const double (&z)[N], const BW64 &c) {
-    bool in_range = true;   // a step moves nu by at most dt/tau |f - nu^a|, so the new nu stays below 1/8 too
+    double tf[N], t[N], p[N], r[N];
+    int in_[N], ie[N];
+    bool in_range = c.dt_itau <= 0.002;   // a step then moves nu too little to leave its centre's series
 #pragma unroll
-    for (int u = 0; u < N; ++u) in_range = in_range && fabs(nu[u] - 1.0) <= 0.12 && fabs(f[u] - 1.0) <= 0.12;
-    if (!(in_range && c.dt_itau <= 0.002)) {
+    for (int u = 0; u < N; ++u) {
+        t[u] = __dmul_rn(c.ln_omr, __dmul_rn(__dsub_rn(1.0, f[u]), rcp_fast(f[u])));
+        ie[u] = exp_index(t[u]);
+        in_[u] = nu_index(nu[u]);
+        in_range = in_range && (unsigned)ie[u] < (unsigned)BW_EXP && (unsigned)in_[u] < (unsigned)BW_NU;
+    }
+    if (!in_range) {
 #pragma unroll
         for (int u = 0; u < N; ++u) bw_step64(x[u], f[u], nu[u], q[u], z[u], c);
         return;
     }
-    double tf[N], inv_f[N], p[N], e[N], y[N], r[N];
+    double2 ct[N];
+    double e[N];
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-        double t = fma(-c.kappa, x[u], z[u]);
-        t = fma(-c.y, __dsub_rn(f[u], 1.0), t);
-        x[u] = fma(c.dt, t, x[u]);
+        ct[u] = __ldg(reinterpret_cast<const double2 *>(c.tab) + in_[u]);
+        e[u] = __ldg(c.tab + 2 * BW_NU + ie[u]);
+        double s = fma(-c.kappa, x[u], z[u]);
+        s = fma(-c.y, __dsub_rn(f[u], 1.0), s);
+        x[u] = fma(c.dt, s, x[u]);
         tf[u] = fma(c.dt, x[u], f[u]);
-        inv_f[u] = rcp_fast(f[u]);
+        e[u] = __dmul_rn(e[u], exp_tiny(fma((double)(BW_EXP0 - ie[u]), 0.125, t[u])));
         p[u] = c.binom[BINOM_TERMS];
-        y[u] = c.ln_omr * ((1.0 - f[u]) * inv_f[u]);
-        e[u] = exp_tiny(y[u]);
     }
 #pragma unroll
     for (int k = BINOM_TERMS - 1; k >= 0; --k)
 #pragma unroll
-        for (int u = 0; u < N; ++u) p[u] = fma(p[u], nu[u] - 1.0, c.binom[k]);
+        for (int u = 0; u < N; ++u) p[u] = fma(p[u], fma(nu[u], ct[u].x, -1.0), c.binom[k]);
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-        nu[u] = fma(c.dt_itau, __dsub_rn(f[u], p[u]), nu[u]);
+        nu[u] = fma(c.dt_itau, __dsub_rn(f[u], __dmul_rn(ct[u].y, p[u])), nu[u]);
         r[u] = rcp_fast(nu[u]);
         p[u] = c.binom[BINOM_TERMS];
     }
 #pragma unroll
     for (int k = BINOM_TERMS - 1; k >= 0; --k)
 #pragma unroll
-        for (int u = 0; u < N; ++u) p[u] = fma(p[u], nu[u] - 1.0, c.binom[k]);
+        for (int u = 0; u < N; ++u) p[u] = fma(p[u], fma(nu[u], ct[u].x, -1.0), c.binom[k]);
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-        const double in = __dmul_rn(__dmul_rn(f[u], __dsub_rn(1.0, c.omr * e[u])), c.irho);
-        const double out = __dmul_rn(__dmul_rn(p[u], q[u]), r[u]);
+        const double in = __dmul_rn(__dmul_rn(f[u], __dsub_rn(1.0, __dmul_rn(c.omr, e[u]))), c.irho);
+        const double out = __dmul_rn(__dmul_rn(__dmul_rn(ct[u].y, p[u]), q[u]), r[u]);
         q[u] = fma(c.dt_itau, __dsub_rn(in, out), q[u]);
         f[u] = tf[u];
     }
