@@ -23,14 +23,15 @@
 //    (8 x 32-bit words per simulation).  The update of bw step m runs during the
 //    GEMMs of bw step m+1 (one simulation pair per inner step), from the inputs
 //    saved at the end of step m, so the FP64 work overlaps the tensor core.  The pair's
-//    two chains overlap (bw_step64_n: 5,172 -> 4,793 cycles a step at 100 nodes); one
+//    two chains overlap (bw_step64_n: 5,172 -> 4,680 cycles a step at 100 nodes); one
 //    simulation per inner step instead of a pair measured 6,180.
 //  * Every wait on the MMA barrier is bounded; on timeout the CTA records a
 //    status, leaves its loop, frees its TMEM and returns.
 //
-// This is the form for large batches; up to 16 simulations per SM integrate_mma.cu's
-// eight-wide tiles are faster (100 nodes, cycles a step of the whole batch: 512 sims
-// 1,900 against 5,172; 2,368 sims 2,650; 4,736 sims 5,250 against 4,793 here).
+// This is the form for large batches of 113-128 nodes; elsewhere integrate_mma.cu's
+// eight-wide tiles are faster (both sides' cycles a step beside the dispatch in
+// session.cpp).  Moving the Balloon-Windkessel model to four warps of its own, as there,
+// left 96 registers a thread and measured 5,387 against 4,678 cycles a step.
 //
 // TMEM columns: [0, NACC TN) accumulator sets | [NACC TN, NACC TN + KP) SC^T hi then lo, two BF16
 // per column, K chunk kk at +8kk | [COLS - 8 TN, COLS) Balloon-Windkessel state.

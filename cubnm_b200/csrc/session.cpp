@@ -1273,10 +1273,13 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         CK(cudaStreamSynchronize(S.st));
     };
     if (use_tc) {
-        // Eight-wide tiles up to 16 simulations per SM (or above 128 nodes), 32-wide above
-        // (100 nodes, cycles per step of the whole batch on 148 SMs: integrate_mma.cu's and
-        // integrate_fp32.cu's header comments).
-        const bool wide = !use_pp && N > 16 * sm_count() && tc32_supported(md.id, n);
+        // Eight-wide tiles, but 32-wide ones for 113-128 nodes and more than 16 simulations
+        // per SM: eight K steps leave the eight-wide kernel too few registers for two CTAs
+        // an SM at full speed.  rWW, cycles a step of the whole batch on 148 SMs, eight-wide
+        // / 32-wide: 128 nodes 8,192 sims 11,489 / 9,407; 100 nodes 2,368 sims 2,178 / 4,678,
+        // 4,736 sims 4,354 / 4,678, 16,384 sims 15,234 / 18,668; 32 nodes 4,736 sims 1,832 /
+        // 4,249; 83 nodes 4,736 sims WC 3,921 / 5,409, JR 5,685 / 7,734.
+        const bool wide = !use_pp && N > 16 * sm_count() && n > 112 && tc32_supported(md.id, n);
         const int TN = use_pp ? 32 : wide ? FP32_TILE_TC : FP32_TILE;
         std::vector<int> tiles = make_tiles(TN);
         if (use_pp) tiles = pair_tiles(tiles, ia.n_tiles, sm_count(), &ia.n_tiles, &ia.pp_grid);
