@@ -195,7 +195,7 @@ cudaError_t launch_integrate_fp64(int model, const IntegrateArgs &a, cudaStream_
 // FP32, eight simulations of one SC per CTA on warp-level matrix products (integrate_mma.cu).
 // Tiles: [n_tiles][1 + FP32_TILE] = SC index, then simulation ids (-1 = empty).
 constexpr int FP32_TILE = 8;
-// FP32, 32 simulations of one SC per CTA on tcgen05 (integrate_fp32.cu): large batches, <= 128 nodes.
+// FP32, 32 simulations of one SC per CTA on tcgen05 (integrate_fp32.cu): large batches of 113-128 nodes.
 constexpr int FP32_TILE_TC = 32;
 bool tc32_supported(int model, int nodes);
 cudaError_t launch_integrate_tc32(int model, const IntegrateArgs &a, cudaStream_t st);
@@ -213,7 +213,7 @@ cudaError_t delay_config32(int model, const IntegrateArgs &a, int sms, DelayLaun
 cudaError_t launch_delay64(int model, const IntegrateArgs &a, const DelayLaunch &c, cudaStream_t st);
 cudaError_t launch_delay32(int model, const IntegrateArgs &a, const DelayLaunch &c, cudaStream_t st);
 cudaError_t launch_integrate_simt32(int model, const IntegrateArgs &a, cudaStream_t st);  // FP32, one CTA per simulation
-// FP32 with 16 simulations on the lanes (integrate_lanes.cu): delays and/or > 128 nodes.
+// FP32 with 16 simulations on the lanes (integrate_lanes.cu): the G tangent; forced or tuned runs.
 bool lanes_supported(int model, int nodes, bool numerical_fic);
 bool lanes_tangent_supported(int model);
 int lanes_rows(int nodes, int threads);
@@ -239,6 +239,7 @@ struct FicArgs {
     const double *gparams;       // [1][n_sims] G
     double *regional;            // [n_regional][n_sims*nodes] (w_p, J_N read; wIE written)
     unsigned char *unstable;     // [n_sims] 1 where FIC failed (wIE set to 1)
+    int round32;                 // wIE rounded to FP32
     RWWK K;
 };
 cudaError_t launch_rww_fic(const FicArgs &a, cudaStream_t st);
@@ -288,6 +289,7 @@ struct AdjArgs {
     double *grad_r;              // [4][n_sims*nodes]  dL/d(w_p, J_N, wIE, sigma)
     int sim_begin, sim_count;    // simulations of this launch (backward: the scratch chunk)
 };
+constexpr int ADJ_REG_NODES = 208;   // most nodes of the adjoint kernels with the SC in registers
 cudaError_t launch_adjoint_forward(const AdjArgs &a, cudaStream_t st);
 cudaError_t launch_adjoint_backward(const AdjArgs &a, cudaStream_t st);
 cudaError_t launch_transpose_sc(const double *sc, float *sc_f32, float *sct_f32, int n_scs, int nodes, cudaStream_t st);

@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(1024) k_rww_fic(const FicArgs a) {
         const double J_N = a.regional[1 * stride + (size_t)sim * n + j];
         const double w = rww_fic_node(sc, n, j, G, w_p, J_N, a.K);
         if (w < 0) bad = 1;
-        a.regional[2 * stride + (size_t)sim * n + j] = w;
+        a.regional[2 * stride + (size_t)sim * n + j] = a.round32 ? (double)(float)w : w;
     }
     bad = __syncthreads_or(bad);
     if (bad)

@@ -11,10 +11,15 @@
 // idle.  Here:
 //
 //  * warp m owns target nodes 16 m .. 16 m + 15 and keeps its rows of SC^T as mma.sync
-//    m16n8k16 A fragments in registers for the whole run (BF16 hi and lo; for more than
-//    176 nodes lo in shared memory); a step loads the eight simulations' x as B
-//    fragments (one 16-byte load per 16 sources brings hi and lo) and issues the BF16x3
-//    products hi hi, hi lo, lo hi into three accumulators, as the tcgen05 kernel does;
+//    m16n8k16 A fragments in registers for the whole run (FP16 hi and lo; for more than
+//    96 nodes lo in shared memory); a step loads the eight simulations' x as B
+//    fragments (one 16-byte load per 16 sources brings hi and lo) and issues the
+//    products hi hi, hi lo, lo hi.  FP16, with each row of SC^T scaled by a power of two
+//    and lo by 2^11, holds 22 bits (x is at most 1 in all four models), so that the sums
+//    are as exact as FP32 ones: BOLD of 40 rWW simulations against FP64, relative, 200
+//    nodes, 2.8e-8 with FP32 sums, 3.2e-8 so; 100 nodes 4.3e-8, 1.2e-7 in BF16 halves
+//    (the tcgen05 form).  The tensor pipe truncates where it accumulates:
+//    hi hi products chained over the K steps gave 9.1e-8, so the FP32 pipe adds them;
 //  * the accumulator layout is the update's layout: lane (g, t) holds nodes g, g + 8 of
 //    the warp and simulations 2t, 2t + 1, state and parameters in registers, stepped as
 //    pairs in packed FP32x2.  K is ordered so that the two nodes of a lane are adjacent
@@ -28,15 +33,17 @@
 //    the node warps its chain of some 300 cycles and its registers cost 545 of 2,240
 //    cycles a step.
 //
-// mma.sync reaches a quarter of tcgen05's rate on sm_100a (measured 950 BF16 multiply-
+// mma.sync reaches a quarter of tcgen05's rate on sm_100a (measured 950 FP16 multiply-
 // adds a cycle and SM), but a tile's 147 products at 100 nodes are 316 cycles of it, in
-// the shadow of the other CTA's update.  Measured at 100 nodes: 1,434 cycles a step with
-// one CTA an SM (8 simulations), 2,178 with two.  What bounds a step then: the phases of a
+// the shadow of the other CTA's update.  Measured at 100 nodes: 1,492 cycles a step with
+// one CTA an SM (8 simulations), 2,262 with two (200 nodes, one: 3,612).  What bounds a step then: the phases of a
 // CTA's warps (product, MUFU, update) follow one another between its barriers, with two
 // CTAs to overlap; more do not fit the registers.
 #include <algorithm>
+#include <cfloat>
 #include <cstdint>
 #include <cstring>
+#include <cuda_fp16.h>
 #include "engine.h"
 #include "tc_common.cuh"
 
@@ -46,11 +53,29 @@ namespace {
 constexpr int TS = 8;            // simulations per tile (MMA N)
 constexpr int NOISE_CHUNK = 10;  // steps of noise per shared-memory buffer (two buffers)
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
     asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+// v = hi + lo / LO_SCALE to 22 bits for 2^-14 <= |v| < 2^15, to 2^-36 below.
+constexpr float LO_SCALE = 2048.0f;
+__device__ __forceinline__ void split_f16x2(float2 v, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __float22half2_rn(v);
+    const float2 hf = __half22float2(h);
+    const __half2 l = __float22half2_rn(__ffma2_rn(hf, make_float2(-LO_SCALE, -LO_SCALE),
+                                                   make_float2(v.x * LO_SCALE, v.y * LO_SCALE)));
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+// The same from zero: the tensor pipe truncates as it accumulates, so that sums of many
+// K steps drift; the hi hi products, which carry it, are added by the FP32 pipe instead.
+__device__ __forceinline__ void mma_f16_add(float2 (&d)[2], const uint4 &a, uint32_t b0, uint32_t b1) {
+    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    mma_f16(c, a, b0, b1);
+    d[0] = __fadd2_rn(d[0], make_float2(c[0], c[1]));
+    d[1] = __fadd2_rn(d[1], make_float2(c[2], c[3]));
 }
 template <int B>
 __device__ __forceinline__ void cp_small(void *dst, const void *src) {
@@ -170,6 +195,7 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
     }
     uint4 ahi[KS], alo[LO_SMEM ? 1 : KS];
     int sc_loaded = -1;
+    float unscale[2] = {1.0f, 1.0f};   // of the rows of its two nodes
 
     for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
         const int *td = a.tiles + (size_t)tile * (TS + 1);
@@ -178,18 +204,31 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
         if (sc_idx != sc_loaded) {
             // K step c, position 2p (+1) of K = source node 16 c + p (+ 8)
             const float *SC = a.sc_f32 + (size_t)sc_idx * n * n;
-            auto w2 = [&](int c, int p, int j, uint32_t &hi, uint32_t &lo) {
+            // a row's weights times the power of two that puts its largest into [2^14, 2^15)
+            float scale[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                float most = 0.0f;
+                if (act[u])
+                    for (int k = t; k < n; k += 4) most = fmaxf(most, fabsf(SC[(size_t)k * n + node[u]]));
+                most = fmaxf(most, __shfl_xor_sync(~0u, most, 1));
+                most = fmaxf(most, __shfl_xor_sync(~0u, most, 2));
+                const int e = most > 0.0f && most <= FLT_MAX ? min(14 - ilogbf(most), 126) : 0;
+                scale[u] = scalbnf(1.0f, e);
+                unscale[u] = scalbnf(1.0f, -e);
+            }
+            auto w2 = [&](int c, int p, int u, uint32_t &hi, uint32_t &lo) {
                 const int k0 = 16 * c + p, k1 = k0 + 8;
-                split_bf16x2(j < n && k0 < n ? SC[(size_t)k0 * n + j] : 0.0f, j < n && k1 < n ? SC[(size_t)k1 * n + j] : 0.0f,
-                             hi, lo);
+                split_f16x2(make_float2(act[u] && k0 < n ? SC[(size_t)k0 * n + node[u]] * scale[u] : 0.0f,
+                                        act[u] && k1 < n ? SC[(size_t)k1 * n + node[u]] * scale[u] : 0.0f), hi, lo);
             };
 #pragma unroll
             for (int c = 0; c < KS; ++c) {
                 uint4 h, l;
-                w2(c, t, node[0], h.x, l.x);
-                w2(c, t, node[1], h.y, l.y);
-                w2(c, t + 4, node[0], h.z, l.z);
-                w2(c, t + 4, node[1], h.w, l.w);
+                w2(c, t, 0, h.x, l.x);
+                w2(c, t, 1, h.y, l.y);
+                w2(c, t + 4, 0, h.z, l.z);
+                w2(c, t + 4, 1, h.w, l.w);
                 ahi[c] = h;
                 if constexpr (LO_SMEM) {
                     alo_s[c * 32] = l;
@@ -224,9 +263,9 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
         // the two nodes' x of simulation 2t and 2t + 1 (padded nodes write 0)
         auto write_x = [&](uint32_t *x) {
             uint32_t h, l;
-            split_bf16x2(act[0] ? s2[0][M::CV].x : 0.0f, act[1] ? s2[1][M::CV].x : 0.0f, h, l);
+            split_f16x2(make_float2(act[0] ? s2[0][M::CV].x : 0.0f, act[1] ? s2[1][M::CV].x : 0.0f), h, l);
             *reinterpret_cast<uint2 *>(x + xw) = make_uint2(h, l);
-            split_bf16x2(act[0] ? s2[0][M::CV].y : 0.0f, act[1] ? s2[1][M::CV].y : 0.0f, h, l);
+            split_f16x2(make_float2(act[0] ? s2[0][M::CV].y : 0.0f, act[1] ? s2[1][M::CV].y : 0.0f), h, l);
             *reinterpret_cast<uint2 *>(x + xw + 16) = make_uint2(h, l);
         };
         // noise of `cnt` steps from inner step i0 of Balloon-Windkessel step b
@@ -256,18 +295,15 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
                 cp_commit();
                 const int i1 = min(i0 + chunk, a.inner_it);
                 for (int inner = i0; inner < i1; ++inner) {
-                    float c[3][4];
-#pragma unroll
-                    for (int s = 0; s < 3; ++s)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) c[s][i] = 0.0f;
+                    float2 hh[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                    float hl[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lh[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
                     for (int k = 0; k < KS; ++k) {   // K steps past the nodes hold zeros
                         const uint4 w = *reinterpret_cast<const uint4 *>(xc + xr + k * 32);
-                        mma_bf16(c[0], ahi[k], w.x, w.z);
-                        mma_bf16(c[1], ahi[k], w.y, w.w);
-                        if constexpr (LO_SMEM) mma_bf16(c[2], alo_s[k * 32], w.x, w.z);
-                        else mma_bf16(c[2], alo[k], w.x, w.z);
+                        mma_f16_add(hh, ahi[k], w.x, w.z);
+                        mma_f16(hl, ahi[k], w.y, w.w);
+                        if constexpr (LO_SMEM) mma_f16(lh, alo_s[k * 32], w.x, w.z);
+                        else mma_f16(lh, alo[k], w.x, w.z);
                     }
                     const float *nz = noise_s + (size_t)(nbuf * chunk + inner - i0) * n * NN;
                     const bool last = inner == a.inner_it - 1;
@@ -281,9 +317,11 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
                             n0 = nz[nzoff[u]];
                         }
                         float2 o[M::NOUT];
-                        Step::step(s2[u], p2[u], make_float2((c[0][2 * u] + c[1][2 * u]) + c[2][2 * u],
-                                                             (c[0][2 * u + 1] + c[1][2 * u + 1]) + c[2][2 * u + 1]),
-                                   n0, n1, K, o);
+                        const float lo_unscale = unscale[u] * (1.0f / LO_SCALE);
+                        const float2 in = __ffma2_rn(make_float2(hl[2 * u] + lh[2 * u], hl[2 * u + 1] + lh[2 * u + 1]),
+                                                     make_float2(lo_unscale, lo_unscale),
+                                                     make_float2(hh[u].x * unscale[u], hh[u].y * unscale[u]));
+                        Step::step(s2[u], p2[u], in, n0, n1, K, o);
                         if (last && sample && act[u]) {
 #pragma unroll
                             for (int w = 0; w < 2; ++w) {

@@ -952,9 +952,9 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         has_delay = *std::max_element(h_max_delay.begin(), h_max_delay.end()) > 0;
     }
     // FP32 kernels: the tensor-core tiles take shared-SC batches without delays or
-    // numerical FIC at <= 224 nodes (200-node rWW, 512 sims: 3,150 cycles a step of the
+    // numerical FIC at <= 224 nodes (200-node rWW, 512 sims: 3,610 cycles a step of the
     // batch against 8,700 on the per-simulation kernel); delayed networks run in blocks of
-    // 32 steps (integrate_delay.cuh: 1,000-node WC, 148 sims: 31,000 cycles per sim-step
+    // 32 steps (integrate_delay.cuh: 1,000-node WC, 148 sims: 19,700 cycles per sim-step
     // and SM against the lane kernel's 66,000), everything else on the per-simulation
     // kernel.  The lane kernel runs the G tangent, and when
     // CBNM_FP32_KERNEL=lanes or the tuner picks it; CBNM_FP32_KERNEL=simt forces the
@@ -1069,6 +1069,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     if (c.do_fic) {
         FicArgs fa;
         fa.nodes = n; fa.n_sims = N; fa.sc = d_sc; fa.sc_idx = d_sc_idx; fa.gparams = d_g; fa.regional = d_r;
+        // as the FP32 per-simulation kernels return it: wIE as integrated
+        fa.round32 = use_tc && n > 128;
         fa.unstable = d_gbools; fa.K = make_constants(MODEL_RWW, c.dt).rww;
         CK(launch_rww_fic(fa, S.st));
     }
@@ -1276,9 +1278,9 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         // Eight-wide tiles, but 32-wide ones for 113-128 nodes and more than 16 simulations
         // per SM: eight K steps leave the eight-wide kernel too few registers for two CTAs
         // an SM at full speed.  rWW, cycles a step of the whole batch on 148 SMs, eight-wide
-        // / 32-wide: 128 nodes 8,192 sims 11,489 / 9,407; 100 nodes 2,368 sims 2,178 / 4,678,
-        // 4,736 sims 4,354 / 4,678, 16,384 sims 15,234 / 18,668; 32 nodes 4,736 sims 1,832 /
-        // 4,249; 83 nodes 4,736 sims WC 3,921 / 5,409, JR 5,685 / 7,734.
+        // / 32-wide: 128 nodes 8,192 sims 11,489 / 9,407; 100 nodes 2,368 sims 2,262 / 4,678,
+        // 4,736 sims 4,511 / 4,678, 16,384 sims 15,765 / 18,668; 32 nodes 4,736 sims 1,888 /
+        // 4,249; 83 nodes 4,736 sims JR 5,682 / 7,734.
         const bool wide = !use_pp && N > 16 * sm_count() && n > 112 && tc32_supported(md.id, n);
         const int TN = use_pp ? 32 : wide ? FP32_TILE_TC : FP32_TILE;
         std::vector<int> tiles = make_tiles(TN);

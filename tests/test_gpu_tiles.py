@@ -107,3 +107,36 @@ def test_fp32_wide_tiles_match_narrow_ones(model, nodes):
     for v in range(wide["_sim_states"].shape[0]):
         scale = max(1.0, float(np.abs(narrow["_sim_states"][v]).max()))
         assert np.abs(wide["_sim_states"][v][pick] - narrow["_sim_states"][v]).max() < 1e-4 * scale, v
+
+
+@pytest.mark.parametrize("model,nodes", [("rWW", 33), ("WC", 97), ("JR", 200)])
+@pytest.mark.parametrize("exponent", [-60, 40])
+def test_fp32_weights_scale_exactly(model, nodes, exponent):
+    """The tiles scale each row of the SC into the range of their 16-bit halves.  A power of
+    two moved from G to the SC changes no bit: every product and sum scales with it."""
+    a = _args(model, nodes, 9, precision="fp32", ms=300)
+    ref = core.run_simulations(*_copy(a))
+    assert core.last_integrator() == "tc1"
+    b = _copy(a)
+    b[1] = b[1] * 2.0 ** exponent
+    b[4] = b[4] * 2.0 ** -exponent
+    got = core.run_simulations(*b)
+    np.testing.assert_array_equal(got["sim_bold"], ref["sim_bold"])
+
+
+@pytest.mark.parametrize("nodes,rounded", [(100, False), (129, True), (224, True), (225, True)])
+def test_fp32_fic_returns_wie_as_integrated(nodes, rounded):
+    """Above 128 nodes an FP32 run returns the wIE of the analytical FIC in FP32, whichever
+    kernel it takes; the solver itself is FP64 in both precisions."""
+    N = 5
+    a = list(cases.synthetic_args("rWW", N=N, nodes=nodes, duration_s=1, seed=nodes, density=0.3,
+                                  G=np.linspace(0.2, 1.2, N), bold_remove_s=0, do_fcd=False, do_fic=1,
+                                  precision="fp64"))
+    a[16], a[17], a[18] = 200, 100, 100
+    wie = []
+    for precision in ("fp64", "fp32"):
+        b = _copy(a)
+        b[7] = dict(a[7], precision=precision)
+        core.run_simulations(*b)
+        wie.append(b[5][2].copy())
+    np.testing.assert_array_equal(wie[1], wie[0].astype(np.float32).astype(np.float64) if rounded else wie[0])
