@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(1024) k_adj_forward(const AdjArgs A) {
             __syncthreads();
             if (act) x1[j] = s[M::CONN];
         }
-        if (act) bw_step64(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bwf);
+        if (act) bw_step(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bw);
         if ((bw_i + 1) % a.bold_tr_iters == 0) {
             if (act && bold_i < a.bold_len)  // no slot for a sample past bold_len
                 bold[(size_t)bold_i * n + j] =
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(1024) k_adj_backward(const AdjArgs A) {
             }
             if (act) {
                 scr_z[(size_t)b * n + j] = s[M::BOLDV];
-                bw_step64(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bwf);
+                bw_step(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bw);
             }
         }
         // ---- reverse through the segment

@@ -10,6 +10,7 @@
 // simulation from t = 0 with adjusted wIE, as the CPU path does.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include "engine.h"
 #include "models.cuh"
 #include "tc_common.cuh"
@@ -51,10 +52,27 @@ struct SimArrays<float> {
 };
 
 // FP32 coupling input of node j, sum_k SC[k][j] x[k] (x in shared memory, 16-byte
-// aligned): sixteen partial sums over k mod 16 (float4 reads of x), combined in the
-// tree of the adjoint kernels' lane butterfly (adjoint.cu), so that both give the same
-// bits.  The FP64 path keeps the reference's sequential order instead.
+// aligned): four independent partial sums over k = 0,1,2,3 mod 4 (float4 reads
+// of x), so the FMA chain is a quarter as long; combined as (s0 + s1) + (s2 + s3).
+// The FP64 path keeps the reference's sequential order instead.
 __device__ __forceinline__ float coupling_f32(const float *__restrict__ SC, const float *x, int n, int j) {
+    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    int k = 0;
+    for (; k + 3 < n; k += 4) {
+        const float4 v = x4[k >> 2];
+        s0 += __ldg(&SC[(size_t)k * n + j]) * v.x;
+        s1 += __ldg(&SC[(size_t)(k + 1) * n + j]) * v.y;
+        s2 += __ldg(&SC[(size_t)(k + 2) * n + j]) * v.z;
+        s3 += __ldg(&SC[(size_t)(k + 3) * n + j]) * v.w;
+    }
+    for (; k < n; ++k) s0 += __ldg(&SC[(size_t)k * n + j]) * x[k];
+    return (s0 + s1) + (s2 + s3);
+}
+
+// The same in sixteen partial sums over k mod 16, combined in the tree of the
+// register-resident adjoint kernels' lane butterfly (adjoint.cu): the same bits as theirs.
+__device__ __forceinline__ float coupling_tree16(const float *__restrict__ SC, const float *x, int n, int j) {
     float p[16];
 #pragma unroll
     for (int l = 0; l < 16; ++l) p[l] = 0.0f;
@@ -82,7 +100,11 @@ __device__ __forceinline__ float coupling_f32(const float *__restrict__ SC, cons
 
 // MAXT = the block size bound: 1024 (at most 64 registers a thread), or 512 (up
 // to 128 registers, no spills) for delayed networks of 129-512 nodes.
-template <class M, bool DELAY, class R, bool SPARSE, int MAXT>
+// ADJ = the sums and the Balloon-Windkessel step of the register-resident adjoint kernels,
+// so that the BOLD is theirs bit for bit.  Elsewhere their registers cost more than they
+// give: WC 300 nodes, 200 sims, 148 ms per simulated second against 85; rWW 390 nodes,
+// 25 %, 123 against 84.
+template <class M, bool DELAY, class R, bool SPARSE, int MAXT, bool ADJ = false>
 __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
     const int sim = a.sim_begin + blockIdx.x;
     const int j = threadIdx.x;
@@ -185,7 +207,7 @@ __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
                         else in += __ldg(&SC[(size_t)k * n + j]) * R(xk);
                     }
                 } else if constexpr (sizeof(R) == 4 && sizeof(S) == 4 && !M::OSC) {
-                    in = coupling_f32(SC, x1, n, j);
+                    in = ADJ ? coupling_tree16(SC, x1, n, j) : coupling_f32(SC, x1, n, j);
                 } else {
                     const S xj = x1[j];
                     for (int k = 0; k < n; ++k) {
@@ -196,7 +218,7 @@ __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
                 const long long ni = ((long long)sh_ts * a.inner_it + inner) * n * M::NN + (long long)sh_j * M::NN;
                 const R n0 = noise[ni];
                 const R n1 = (M::NN > 1) ? noise[ni + 1] : R(0);
-                M::step(s, iv, g, r, in, n0, n1, a.K);
+                M::template step<sizeof(R) == 8>(s, iv, g, r, in, n0, n1, a.K);
             }
             __syncthreads();  // every read of the previous conn-states is done
             if (act) {
@@ -206,7 +228,7 @@ __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
             if (DELAY) buff = (buff + D - 1) % D;
         }
         if (act) {
-            if constexpr (sizeof(R) == 4) bw_step64(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bwf);
+            if constexpr (ADJ) bw_step64(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bwf);
             else bw_step(bx, bf, bnu, bq, (double)s[M::BOLDV], a.bw);
         }
         if ((bw_i + 1) % a.bold_tr_iters == 0) {  // bnm.cpp:316-335
@@ -322,6 +344,12 @@ cudaError_t launch_sim_kernel(const IntegrateArgs &a, cudaStream_t st) {
     const int threads = ((a.nodes + 31) / 32) * 32;
     const size_t smem = a.has_delay ? 0 : sizeof(typename M::S) * a.nodes;
     const int grid = a.n_sims - a.sim_begin;
+    if constexpr (std::is_same<M, RWWm<float>>::value) {
+        if (!a.has_delay && a.ell_k == 0 && !a.do_fic && a.nodes <= ADJ_REG_NODES) {
+            k_integrate_sim<M, false, R, false, 1024, true><<<grid, threads, smem, st>>>(a);
+            return cudaGetLastError();
+        }
+    }
     if (!a.has_delay) return launch_sim_variant<M, R, 1024, false>(a, grid, threads, smem, st);
     if constexpr (UNCAP) {
         if (threads > 128 && threads <= 512) return launch_sim_variant<M, R, 512, true>(a, grid, threads, smem, st);

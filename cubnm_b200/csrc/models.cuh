@@ -60,6 +60,14 @@ __device__ __forceinline__ float rate_of(float x, float d) {
     return zero ? 1.0f / d : div_nr(x, zero ? 1.0f : -expm1f(y));
 }
 
+// IEEE: with the division operator.  The per-simulation FP64 kernel, at 64 registers a
+// thread, takes it (rWW, 160 nodes, 300 sims: 44.4 ms per simulated second against 46.5).
+template <bool IEEE, class R>
+__device__ __forceinline__ R rate(R x, R d) {
+    if constexpr (IEEE) return x / (1 - exp(-d * x));
+    else return rate_of(x, d);
+}
+
 template <class R>
 struct RWWm {
     using S = R;
@@ -71,15 +79,15 @@ struct RWWm {
         s[4] = R(0.001); s[5] = R(0.001);
     }
     __device__ static void restart(S *s, R *, const P *) { s[4] = R(0.001); s[5] = R(0.001); }
-    template <class KK>
+    template <bool IEEE_DIV = false, class KK>
     __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R n1, const KK &K) {  // rww.cpp:194-232
         const auto &m = K.rww;
         s[0] = R(m.w_E__I_0) + r[0] * r[1] * s[4] + in * g[0] * r[1] - r[2] * s[5];
         s[1] = R(m.w_I__I_0) + r[1] * s[4] - R(m.w_II) * s[5];
         iv[0] = R(m.a_E) * s[0] - R(m.b_E);
         iv[1] = R(m.a_I) * s[1] - R(m.b_I);
-        s[2] = rate_of(iv[0], R(m.d_E));
-        s[3] = rate_of(iv[1], R(m.d_I));
+        s[2] = rate<IEEE_DIV>(iv[0], R(m.d_E));
+        s[3] = rate<IEEE_DIV>(iv[1], R(m.d_I));
         iv[2] = n0 * r[3] * R(m.sqrt_dt) + R(m.dt_gamma_E) * ((R(1) - s[4]) * s[2]) - R(m.dt_itau_E) * s[4];
         iv[3] = n1 * r[3] * R(m.sqrt_dt) + R(m.dt_gamma_I) * s[3] - R(m.dt_itau_I) * s[5];
         s[4] += iv[2];
@@ -97,7 +105,7 @@ struct WCm {
     static constexpr bool OSC = false, POSTBW = false;
     __device__ static void init(S *s, R *, const R *, const P *) { s[0] = R(0.001); s[1] = R(0.001); }
     __device__ static void restart(S *s, R *, const P *) { s[0] = R(0.001); s[1] = R(0.001); }
-    template <class KK>
+    template <bool IEEE_DIV = false, class KK>
     __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R n1, const KK &K) {  // wc.cpp:51-80
         const auto &m = K.wc;
         iv[0] = R(1) / (R(1) + exp(-R(m.a_E) * (r[0] * s[0] - r[1] * s[1] + g[0] * in + r[4] - R(m.mu_E))));
@@ -121,7 +129,7 @@ struct JRm {
         for (int i = 0; i < 8; ++i) s[i] = R(0);
     }
     __device__ static void restart(S *s, R *, const P *) { for (int i = 0; i < 8; ++i) s[i] = R(0); }
-    template <class KK>
+    template <bool IEEE_DIV = false, class KK>
     __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const KK &K) {  // jr.cpp:80-133
         const auto &m = K.jr;
         iv[0] = R(2) * R(m.nu_max) / (R(1) + exp(R(m.r) * (R(m.v0) - (s[1] - s[2]))));
@@ -152,7 +160,7 @@ struct Kuramotom {
     static constexpr bool OSC = true, POSTBW = false;
     __device__ static void init(S *s, R *, const R *, const P *r) { s[0] = S(r[0]); }
     __device__ static void restart(S *s, R *, const P *r) { s[0] = S(r[0]); }
-    template <class KK>
+    template <bool IEEE_DIV = false, class KK>
     __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const KK &K) {  // kuramoto.cpp:48-61
         const auto &m = K.kur;
         const S w = r[1] + S(g[0] * in);  // instantaneous frequency, in double
@@ -170,12 +178,12 @@ struct RWWExm {
     static constexpr bool OSC = false, POSTBW = false;
     __device__ static void init(S *s, R *, const R *, const P *) { s[0] = s[1] = R(0); s[2] = R(0.001); }
     __device__ static void restart(S *s, R *, const P *) { s[2] = R(0.001); }
-    template <class KK>
+    template <bool IEEE_DIV = false, class KK>
     __device__ static void step(S *s, R *iv, const R *g, const P *r, R in, R n0, R, const KK &K) {  // rwwex.cpp:48-73
         const auto &m = K.rwwex;
         s[0] = r[0] * R(m.J_N) * s[2] + g[0] * R(m.J_N) * in + r[1];
         iv[0] = R(m.a) * s[0] - R(m.b);
-        s[1] = rate_of(iv[0], R(m.d));
+        s[1] = rate<IEEE_DIV>(iv[0], R(m.d));
         iv[1] = R(m.dt_gamma) * ((R(1) - s[2]) * s[1]) - R(m.dt_itau) * s[2] + n0 * R(m.sqrt_dt) * r[2];
         s[2] += iv[1];
         s[2] = fmax(R(0), fmin(R(1), s[2]));
