@@ -1,4 +1,7 @@
-// FP64 integrator: the reference-precision path (the "plain" GPU method).
+// FP64 per-simulation integrator: the reference-precision kernel for what
+// integrate_tile64.cu (up to 128 nodes without delays) and integrate_delay.cuh (delays) do
+// not take -- Kuramoto, numerical FIC, more than 128 nodes without delays, forced coupling
+// forms.
 //
 // The per-simulation kernel of integrate_sim.cuh with R = double: one CTA per
 // simulation, one thread per node, everything in FP64, so that its output

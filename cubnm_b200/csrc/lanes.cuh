@@ -1,9 +1,10 @@
-// FP32 integrator with the simulations on the lanes, for the networks the
-// tensor-core tiles do not take: conduction delays (any node count) and more than
-// 128 nodes.  The time loop is the reference's (src/ext/bnm.cu:117-505); the
+// FP32 integrator with the simulations on the lanes: the G tangent, and forward runs
+// where it is forced or the autotuner picks it (networks with conduction delays of any
+// node count, or of more than 128 nodes; by default those take integrate_delay.cuh and
+// integrate_mma.cu, which measured faster).  The time loop is the reference's (src/ext/bnm.cu:117-505); the
 // delayed coupling is bnm.cu:48-77 with the ring-buffer index of bnm.cu:28-46.
 //
-// The per-simulation kernel (integrate_sim.cuh, the reference's one CTA per
+// The per-step kernel (integrate_sim.cuh, the reference's one CTA per
 // simulation and one thread per node) gathers x_k(t - d_kj) from the
 // simulation's own ring buffer: each 4-byte value costs a 32-byte sector, and
 // every simulation re-reads the SC / delay entries.  Here 16 simulations that

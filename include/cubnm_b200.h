@@ -187,9 +187,10 @@ int cbnm_reset(void);
 const char *cbnm_last_error(void);
 
 /* Integrator of the last run on this thread: "fp64", or for precision "fp32"
- * "tc2" (two-tile tensor-core kernel), "tc1" (single-tile tensor-core kernel),
+ * "tc2" / "tc2ws" (two-tile tensor-core kernel), "tc1" (one-tile kernels: eight
+ * simulations on warp matrix products or 32 on tcgen05),
  * "lanes" / "lanes512" (simulations on the lanes, 1024 / 512 threads a CTA) or
- * "simt" (one CTA per simulation).  No reference counterpart (diagnostic). */
+ * "simt" (one CTA per simulation, delayed networks in blocks of steps).  No reference counterpart (diagnostic). */
 const char *cbnm_last_integrator(void);
 
 /* FP32 fused-multiply-add throughput of the current device in TFLOP/s (two flops

@@ -94,7 +94,7 @@ def test_steps_per_millisecond(precision, dt):
 @pytest.mark.parametrize("model,nodes", [("rWW", 113), ("rWW", 128), ("WC", 128), ("JR", 120), ("rWWEx", 127)])
 def test_fp32_wide_tiles_match_narrow_ones(model, nodes):
     """More than 16 simulations per SM of 113-128 nodes take the 32-wide tcgen05 tiles; the
-    same simulations alone the eight-wide ones.  Both form the coupling in BF16x3 with FP32 sums."""
+    same simulations alone the eight-wide ones.  Both form the coupling from 16-bit halves with FP32 sums."""
     N = 2500
     a = _args(model, nodes, N, precision="fp32", ms=300)
     a[1] = np.stack([cases.synthetic_sc(nodes, 0.6, s).reshape(-1) for s in (1, 2)])
