@@ -44,20 +44,20 @@ DURATION_S = 60
 # dram__bytes_read.sum + dram__bytes_write.sum of one integrator launch of the default
 # workload, from an ncu capture of one launch on a reduced case scaled by the
 # simulated node-steps (profiles/ names the capture); None until measured
-TRAFFIC_DEFAULT_WORKLOAD = 6.242e9
-TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_integrate_tc launch on 9,472 sims x "
-                  "8 s (240.6 MB), scaled by node-steps to 32,768 x 60 s "
-                  "(profiles/k_integrate_tc_rww_9472x8s_counters.md)")
+TRAFFIC_DEFAULT_WORKLOAD = 11.49e9
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_integrate_mma launch on 9,472 sims x "
+                  "8 s (442.9 MB), scaled by node-steps to 32,768 x 60 s "
+                  "(profiles/k_integrate_mma_rww_9472x8s_dram.md)")
 # FP32 flops of one rWW node update (rww.cpp:194-232): I_E 8, I_I 4, the two affine
 # rate arguments 4, the two rates (without their exp) 6, dS_E 8, dS_I 6, the two
 # state additions 2
 RWW_FP32_FLOPS = 38
 WORKLOAD = f"rWW {NODES} nodes, {N_SIMS} sims, {DURATION_S} s, dt 0.1 ms, TR 1 s, FC+FCD w10/s2"
 # the kernel behind each integrator name of core.last_integrator()
-KERNEL_OF = {"tc1": "k_integrate_tc<RWW32, Tile<32, 8, 3>>", "tc2": "k_integrate_pp<RWW32>",
-             "tc2ws": "k_integrate_pp_ws<RWW32>", "simt": "k_integrate_sim<M, delay, float>",
+KERNEL_OF = {"tc1": "k_integrate_mma<M, ceil(nodes / 16)>", "tc2": "k_integrate_pp<RWW32>",
+             "tc2ws": "k_integrate_pp_ws<RWW32>", "simt": "k_integrate_delay<M, float>",
              "lanes": "k_integrate_lanes<M, 1024, ...>", "lanes512": "k_integrate_lanes<M, 512, ...>",
-             "fp64": "k_integrate_sim<M, delay, double>"}
+             "fp64": "k_tile64<M> (k_integrate_delay<M, double> with delays)"}
 METRIC = "rWW sims x sim-s per wall-s (100 nodes, 32k sims)"
 UNIT = "sims*sim-s/s"
 
@@ -276,11 +276,11 @@ def run_ours(opts, rank, world, local_rank):
     node_steps = n_sims * NODES * (opts.duration * 1000 / 0.1)
     integ = float(np.mean(integ_ms)) / 1e3
     useful = 2.0 * NODES * node_steps  # coupling flops (2 n per node-step)
-    issued = 3 * 2.0 * 128 * (((NODES + 15) // 16) * 16) * (n_sims * 1.0) * (opts.duration * 1e4)  # BF16x3 MMA work
+    issued = 3 * 2.0 * (((NODES + 15) // 16) * 16) ** 2 * n_sims * (opts.duration * 1e4)  # hi / lo MMA work
     fp32_flops = RWW_FP32_FLOPS * node_steps
     traffic, traffic_src = opts.traffic, "--traffic" if opts.traffic is not None else None
     if (traffic is None and n_sims == N_SIMS and opts.duration == DURATION_S and opts.precision == "fp32"
-            and integrator == "tc1"):  # the capture is of the single-tile kernel
+            and integrator == "tc1"):  # the capture is of the eight-wide tiles
         traffic, traffic_src = TRAFFIC_DEFAULT_WORKLOAD, TRAFFIC_SOURCE
     roof = {"bound": "fp32", "achieved": fp32_flops / integ / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
             "frac": fp32_flops / integ / 1e12 / fp32_peak,
@@ -300,7 +300,7 @@ def run_ours(opts, rank, world, local_rank):
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": opts.steps,
         "warmup": opts.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f32 (BF16x3 tensor-core coupling, FP64 Balloon-Windkessel and FC/FCD)",
+        "vs_baseline": None, "dtype": "f32 (tensor-core coupling in FP16 hi + lo, FP64 Balloon-Windkessel and FC/FCD)",
         "data": "synthetic (seeded SC, parameters and noise)",
         "config": {"workload": WORKLOAD, "sims_per_gpu": n_sims, "nodes": NODES, "duration_s": opts.duration,
                    "precision": opts.precision, "parallelism": f"independent sims x{world}",
@@ -513,7 +513,8 @@ def config_roofline(args, integrate_ms, delayed, fp32_peak=None):
         return {"bound": "hbm", "achieved": b / t / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": b / t / 1e9 / peaks["hbm_gbs"], "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
                 "traffic": None, "algorithmic_bytes": b,
-                "work": f"{nnz:.1f} ring-buffer gathers x 4 B per node-step, {node_steps:.3e} node-steps",
+                "work": f"{nnz:.1f} ring-buffer gathers x 4 B per node-step (from shared memory, where the "
+                        f"delay kernel stages the buffers every 32 steps), {node_steps:.3e} node-steps",
                 "kernel": kernel, "kernel_ms": integrate_ms}
     flops = node_steps * (2.0 * nnz + RWW_FP32_FLOPS)
     return {"bound": "fp32", "achieved": flops / t / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
@@ -538,7 +539,8 @@ def batch_roofline(groups, seconds):
     return {"bound": "hbm", "achieved": b / seconds / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": b / seconds / 1e9 / peaks["hbm_gbs"], "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
             "traffic": None, "algorithmic_bytes": b,
-            "work": "ring-buffer gathers of every group, 4 B per nonzero per node-step",
+            "work": "ring-buffer gathers of every group, 4 B per nonzero per node-step (from shared memory, where "
+                    "the delay kernel stages the buffers every 32 steps)",
             "basis": "whole-batch wall time (the groups' kernels run concurrently on their own streams)"}
 
 
