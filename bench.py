@@ -53,11 +53,6 @@ TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_int
 # state additions 2
 RWW_FP32_FLOPS = 38
 WORKLOAD = f"rWW {NODES} nodes, {N_SIMS} sims, {DURATION_S} s, dt 0.1 ms, TR 1 s, FC+FCD w10/s2"
-# the kernel behind each integrator name of core.last_integrator()
-KERNEL_OF = {"tc1": "k_integrate_mma<M, ceil(nodes / 16)>", "tc2": "k_integrate_pp<RWW32>",
-             "tc2ws": "k_integrate_pp_ws<RWW32>", "simt": "k_integrate_delay<M, float>",
-             "lanes": "k_integrate_lanes<M, 1024, ...>", "lanes512": "k_integrate_lanes<M, 512, ...>",
-             "fp64": "k_tile64<M> (k_integrate_delay<M, double> with delays)"}
 METRIC = "rWW sims x sim-s per wall-s (100 nodes, 32k sims)"
 UNIT = "sims*sim-s/s"
 
@@ -206,7 +201,7 @@ def run_ours(opts, rank, world, local_rank):
     e1.record(st)
     barrier()
     ck = clocks.stop()
-    integrator = core.last_integrator()
+    integrator, kernel = core.last_integrator(), core.last_kernel()
     ms = max_over_ranks(e0.elapsed_time(e1) / opts.steps)
     value = world * n_sims * opts.duration / (ms / 1e3)
 
@@ -280,7 +275,7 @@ def run_ours(opts, rank, world, local_rank):
     fp32_flops = RWW_FP32_FLOPS * node_steps
     traffic, traffic_src = opts.traffic, "--traffic" if opts.traffic is not None else None
     if (traffic is None and n_sims == N_SIMS and opts.duration == DURATION_S and opts.precision == "fp32"
-            and integrator == "tc1"):  # the capture is of the eight-wide tiles
+            and kernel == "k_integrate_mma"):  # the captured kernel
         traffic, traffic_src = TRAFFIC_DEFAULT_WORKLOAD, TRAFFIC_SOURCE
     roof = {"bound": "fp32", "achieved": fp32_flops / integ / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
             "frac": fp32_flops / integ / 1e12 / fp32_peak,
@@ -294,7 +289,7 @@ def run_ours(opts, rank, world, local_rank):
                        "mma_issued_tflops": issued / integ / 1e12},
             "traffic": traffic, "traffic_source": traffic_src,
             "algorithmic_bytes": N_SIMS * NODES * DURATION_S * 8.0 if n_sims == N_SIMS else None,
-            "kernel": KERNEL_OF.get(integrator, integrator), "kernel_ms": integ * 1e3,
+            "kernel": kernel, "kernel_ms": integ * 1e3,
             "note": "per-pipe utilisation of this kernel: profiles/ (ncu)"}
 
     line = {
@@ -506,7 +501,7 @@ def config_roofline(args, integrate_ms, delayed, fp32_peak=None):
     nnz = float(np.count_nonzero(sc[np.asarray(args[2], dtype=int)])) / (N * n)  # mean nonzeros per target
     node_steps = N * n * (args[16] / args[20])
     t = integrate_ms / 1e3
-    kernel = KERNEL_OF.get(core.last_integrator(), core.last_integrator())
+    kernel = core.last_kernel()
     if delayed:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
         b = node_steps * nnz * 4.0

@@ -84,6 +84,16 @@ def last_integrator():
     return f().decode()
 
 
+def last_kernel():
+    """The CUDA kernel behind :func:`last_integrator`: "k_one64", "k_tile64",
+    "k_integrate_mma", "k_integrate_tc", "k_integrate_pp", "k_integrate_pp_ws",
+    "k_integrate_delay" ("k_integrate_delay/2" with two passes over the targets),
+    "k_integrate_lanes" or "k_integrate_sim"."""
+    f = lib().cbnm_last_kernel
+    f.restype = C.c_char_p
+    return f().decode()
+
+
 def tune_reset():
     """Forgets the autotuner's choices (model_config "autotune" = "1")."""
     check(lib().cbnm_tune_reset())

@@ -712,6 +712,7 @@ static std::map<std::string, int> g_tuned;
 static bool g_tune_loaded = false;
 static Session *g_tune = nullptr;                     // probes run on a session of their own
 static thread_local std::string t_last_variant = "";
+static thread_local std::string t_last_kernel = "";   // the kernel behind it
 
 static int variant_of(const std::string &name) {
     for (int v = 0; v < V_COUNT; ++v)
@@ -1274,6 +1275,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         ia.tiles = S.d_tiles.as<int>();
         CK(cudaStreamSynchronize(S.st));
     };
+    bool tc_wide = false;
     if (use_tc) {
         // Eight-wide tiles, but 32-wide ones for 113-128 nodes and more than 16 simulations
         // per SM: eight K steps leave the eight-wide kernel too few registers for two CTAs
@@ -1281,8 +1283,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         // / 32-wide: 128 nodes 8,192 sims 11,489 / 9,407; 100 nodes 2,368 sims 2,262 / 4,678,
         // 4,736 sims 4,511 / 4,678, 16,384 sims 15,765 / 18,668; 32 nodes 4,736 sims 1,888 /
         // 4,249; 83 nodes 4,736 sims JR 5,682 / 7,734.
-        const bool wide = !use_pp && N > 16 * sm_count() && n > 112 && tc32_supported(md.id, n);
-        const int TN = use_pp ? 32 : wide ? FP32_TILE_TC : FP32_TILE;
+        tc_wide = !use_pp && N > 16 * sm_count() && n > 112 && tc32_supported(md.id, n);
+        const int TN = use_pp ? 32 : tc_wide ? FP32_TILE_TC : FP32_TILE;
         std::vector<int> tiles = make_tiles(TN);
         if (use_pp) tiles = pair_tiles(tiles, ia.n_tiles, sm_count(), &ia.n_tiles, &ia.pp_grid);
         ia.pp_ws = pp_ws ? 1 : 0;
@@ -1291,7 +1293,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         CK(cudaEventRecord(S.ev[1], S.st));
         if (use_pp) CK(launch_integrate_pp(md.id, ia, S.st, &launches));
         else {
-            CK((wide ? launch_integrate_tc32 : launch_integrate_mma)(md.id, ia, S.st));
+            CK((tc_wide ? launch_integrate_tc32 : launch_integrate_mma)(md.id, ia, S.st));
             ++launches;
         }
     } else if (use_lanes) {
@@ -1376,6 +1378,11 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         ++launches;
     }
     t_last_variant = !c.fp32 ? "fp64" : use_pp ? (pp_ws ? "tc2ws" : "tc2") : use_tc ? "tc1" : use_lanes ? (lanes_threads == 512 ? "lanes512" : "lanes") : "simt";
+    t_last_kernel = use_pp ? (pp_ws ? "k_integrate_pp_ws" : "k_integrate_pp")
+                    : use_tc ? (tc_wide ? "k_integrate_tc" : "k_integrate_mma")
+                    : use_lanes ? "k_integrate_lanes"
+                    : delay_blocks ? (plan.passes == 2 ? "k_integrate_delay/2" : "k_integrate_delay")
+                    : t64 ? (t64_tiles ? "k_tile64" : "k_one64") : "k_integrate_sim";
     CK(cudaEventRecord(S.ev[2], S.st));
     if (!device_io) {  // the integrator runs asynchronously: map the host output pages meanwhile
         prefault_host(o->sim_bold, sizeof(double) * bold_n);
@@ -1857,6 +1864,8 @@ int cbnm_reset(void) {
 const char *cbnm_last_error(void) { return g_err.c_str(); }
 
 const char *cbnm_last_integrator(void) { return t_last_variant.c_str(); }
+
+const char *cbnm_last_kernel(void) { return t_last_kernel.c_str(); }
 
 int cbnm_measure_fp32_peak(double *ffma_tflops, double *ffma2_tflops) {
     return guarded([&] {

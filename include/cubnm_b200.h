@@ -193,6 +193,12 @@ const char *cbnm_last_error(void);
  * "simt" (one CTA per simulation, delayed networks in blocks of steps).  No reference counterpart (diagnostic). */
 const char *cbnm_last_integrator(void);
 
+/* CUDA kernel of that run: "k_one64", "k_tile64", "k_integrate_mma", "k_integrate_tc",
+ * "k_integrate_pp", "k_integrate_pp_ws", "k_integrate_delay" ("k_integrate_delay/2": two
+ * passes over the targets), "k_integrate_lanes" or "k_integrate_sim".  No reference
+ * counterpart (diagnostic). */
+const char *cbnm_last_kernel(void);
+
 /* FP32 fused-multiply-add throughput of the current device in TFLOP/s (two flops
  * a lane per FMA), scalar and packed two-wide: the measured denominator of the
  * integrators' FP32 roofline.  Takes about a quarter of a second.  No reference

@@ -1,0 +1,48 @@
+"""Which kernel integrates a run, by its sizes (core.last_kernel)."""
+import numpy as np
+import pytest
+
+import cases
+from cubnm_b200 import core
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(model, nodes, N, precision, velocity=0.0, density=0.3, **config):
+    a = list(cases.synthetic_args(model, N=N, nodes=nodes, duration_s=1, seed=nodes, density=density,
+                                  G=np.linspace(0.2, 1.2, N), bold_remove_s=0, do_fcd=False, precision=precision))
+    a[7] = dict(a[7], do_fc="0", noise_time_steps="100", **config)
+    a[16], a[17], a[18] = 100, 100, 100
+    if velocity:
+        a[3] = np.ascontiguousarray(cases.synthetic_lengths(nodes, nodes).ravel())
+        a[6] = np.full(N, velocity)
+        a[11] = True
+    core.run_simulations(*a)
+    return core.last_kernel()
+
+
+@pytest.mark.parametrize("model,nodes,N,precision,kernel", [
+    ("rWW", 68, 5, "fp64", "k_one64"), ("rWW", 128, 1200, "fp64", "k_tile64"), ("rWW", 129, 5, "fp64", "k_integrate_sim"),
+    ("Kuramoto", 40, 5, "fp64", "k_integrate_sim"), ("rWW", 100, 5000, "fp32", "k_integrate_mma"),
+    ("WC", 128, 100, "fp32", "k_integrate_mma"), ("WC", 128, 2500, "fp32", "k_integrate_tc"),
+    ("JR", 200, 9, "fp32", "k_integrate_mma"), ("rWW", 225, 9, "fp32", "k_integrate_sim")])
+def test_without_delays(model, nodes, N, precision, kernel):
+    assert _run(model, nodes, N, precision) == kernel
+
+
+@pytest.mark.parametrize("model,nodes,precision,density,kernel", [
+    ("rWW", 100, "fp64", 0.2, "k_integrate_delay"), ("WC", 400, "fp32", 0.2, "k_integrate_delay"),
+    ("rWW", 1000, "fp32", 0.1, "k_integrate_delay/2"), ("rWW", 600, "fp64", 0.2, "k_integrate_delay"),
+    ("rWW", 900, "fp64", 0.1, "k_integrate_sim"), ("Kuramoto", 60, "fp64", 0.2, "k_integrate_sim")])
+def test_with_delays(model, nodes, precision, density, kernel):
+    assert _run(model, nodes, 3, precision, velocity=6.0, density=density) == kernel
+
+
+def test_forced_kernels(monkeypatch):
+    monkeypatch.setenv("CBNM_FP32_KERNEL", "simt")
+    assert _run("rWW", 100, 20, "fp32") == "k_integrate_sim"
+    monkeypatch.setenv("CBNM_FP32_KERNEL", "lanes")
+    assert _run("rWW", 150, 20, "fp32", velocity=6.0) == "k_integrate_lanes"
+    monkeypatch.delenv("CBNM_FP32_KERNEL")
+    monkeypatch.setenv("CBNM_FP32_TC", "pp")
+    assert _run("rWW", 100, 100, "fp32") == "k_integrate_pp"
