@@ -39,6 +39,8 @@ constexpr int BW_NU = 17, BW_NU0 = 8, BW_EXP = 20, BW_EXP0 = 16;
 struct BWFast {
     double dt, kappa, y, dt_itau, ialpha, irho, log2_omr, ln_omr, omr, V0k1, V0k2, V0k3;
     double binom[13];            // C(1/alpha, k), k = 0..12
+    int reach;                   // bw_step64_n: bound on f / nu, as a difference of their high words
+    int nu_end;                  // and on nu's table index
     const double *tab;           // device: {c^-1, c^(1/alpha)} for c = 1.25^(i - BW_NU0), then e^((i - BW_EXP0) / 8)
 };
 

@@ -65,7 +65,7 @@ struct Smem {
 
 // ---------------------------------------------------------------- kernel
 template <class M>
-__global__ void __launch_bounds__(NTHREADS, 1) k_integrate_tc(const IntegrateArgs a, const int *tiles, int n_tiles, int KP) {
+__global__ void __launch_bounds__(NTHREADS, 1) k_integrate_tc(const __grid_constant__ IntegrateArgs a, const int *tiles, int n_tiles, int KP) {
     constexpr int COL_A = TN * NACC;                   // A_hi at COL_A, A_lo at COL_A + KP/2 (bf16 pairs)
     constexpr int COL_BWT = TMEM_COLS - TN * 8;        // Balloon-Windkessel state at the top
     extern __shared__ __align__(1024) uint8_t smem_raw[];

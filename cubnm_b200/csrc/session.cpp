@@ -86,6 +86,16 @@ static void fill_bwf(IntegrateArgs &ia, const double *tab) {
     f.irho = 1.0 / ia.bw.rho; f.log2_omr = std::log2(ia.bw.oneminrho); f.ln_omr = std::log(ia.bw.oneminrho);
     f.omr = ia.bw.oneminrho;
     f.V0k1 = ia.bw.V_0 * ia.bw.k1; f.V0k2 = ia.bw.V_0 * ia.bw.k2; f.V0k3 = ia.bw.V_0 * ia.bw.k3;
+    // A step moves nu by dt_itau (f - nu^(1/alpha)).  Both terms at most 0.0105 c: a centre's
+    // edges are 1.25^(+-1/2) (nu / c from 0.894 to 1.118), and with that nu / c stays within
+    // 0.1289 of 1.  High words are 2^20 log2, less up to 0.087 2^20.
+    f.reach = (int)std::floor((std::log2(0.0105 / 1.119 / f.dt_itau) - 0.087) * (1 << 20));
+    f.nu_end = 0;
+    while (f.nu_end < BW_NU) {
+        const double centre = std::pow(1.25, f.nu_end - BW_NU0), top = centre * 1.119;
+        if (f.dt_itau * std::pow(top, f.ialpha) > 0.0105 * centre) break;
+        ++f.nu_end;
+    }
     long double v = 1.0L;   // C(1/alpha, k) for the binomial form of nu^(1/alpha)
     f.binom[0] = 1.0;
     for (int k = 1; k <= 12; ++k) {

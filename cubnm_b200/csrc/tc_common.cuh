@@ -399,19 +399,24 @@ __device__ __forceinline__ double pow_omr(double f, double inv_f, const BW64 &c)
 
 // Every multiply-add below is spelled out (fma / __dmul_rn / __dadd_rn), so the
 // compiler's contraction choices, which can differ between the kernels this is
-// inlined into, never change a bit of the result: the same inputs give the same
-// BOLD in every integrator that uses it.
-__device__ __forceinline__ void bw_step64(double &x, double &f, double &nu, double &q, double z, const BW64 &c) {
-    double t = fma(-c.kappa, x, z);
-    t = fma(-c.y, __dsub_rn(f, 1.0), t);
-    x = fma(c.dt, t, x);
-    const double tmp_f = fma(c.dt, x, f);
-    const double inv_f = rcp_fast(f);
-    nu = fma(c.dt_itau, __dsub_rn(f, pow_nu(nu, c)), nu);
-    const double in = __dmul_rn(__dmul_rn(f, __dsub_rn(1.0, pow_omr(f, inv_f, c))), c.irho);
-    const double out = __dmul_rn(__dmul_rn(pow_nu(nu, c), q), rcp_fast(nu));
-    q = fma(c.dt_itau, __dsub_rn(in, out), q);
-    f = tmp_f;
+// inlined into, never change a bit of the result.
+//
+// The general form, for states outside the table: exp2 / log2 powers and IEEE division.
+// Out of line, so that it costs the usual form no registers.
+struct BWState { double x, f, nu, q; };
+__device__ __noinline__ double bw_pow_any(double nu, double ialpha) { return exp2(ialpha * log2(nu)); }
+__device__ __noinline__ BWState bw_step64_any(BWState s, double z, double dt, double kappa, double y, double dt_itau,
+                                              double ialpha, double irho, double log2_omr) {
+    double t = fma(-kappa, s.x, z);
+    t = fma(-y, __dsub_rn(s.f, 1.0), t);
+    s.x = fma(dt, t, s.x);
+    const double f0 = s.f;
+    s.f = fma(dt, s.x, f0);
+    s.nu = fma(dt_itau, __dsub_rn(f0, bw_pow_any(s.nu, ialpha)), s.nu);
+    const double in = __dmul_rn(__dmul_rn(f0, __dsub_rn(1.0, exp2(__ddiv_rn(log2_omr, f0)))), irho);
+    const double out = __ddiv_rn(__dmul_rn(bw_pow_any(s.nu, ialpha), s.q), s.nu);
+    s.q = fma(dt_itau, __dsub_rn(in, out), s.q);
+    return s;
 }
 
 // BOLD = V0 (k1 (1 - q) + k2 (1 - q / nu) + k3 (1 - nu))  (bnm.cpp:316-335)
@@ -421,27 +426,74 @@ __device__ __forceinline__ double bold64(double q, double nu, const BW64 &c) {
     return fma(c.V0k3, __dsub_rn(1.0, nu), b);
 }
 
-// The step of N items.  Where all are within the table there is no branch, so the items'
-// chains of dependent FP64 operations overlap: with the range tests of bw_step64 inside,
-// two items took 2,700 cycles one after the other in the tile kernel.  The same
-// operations, but the new nu is expanded around the old one's centre, so results differ
-// from bw_step64 in the last bits at a step where nu passes between centres.
+// Whether the new nu, d = nu / c - 1 in units of the old one's centre c, is within reach of
+// that centre's series for the second power of the step: |d| < 0.1289 (high words
+// compared; a centre is within 0.1185), where the first omitted term, C(1/alpha, 13) d^13, is below 1e-16.
+__device__ __forceinline__ bool bw_in_reach(double d) { return (__double2hiint(d) & 0x7fffffff) <= 0x3fc08000; }
+
+// One step.  The new nu is expanded around the old one's centre, or its power taken from
+// the general form where the step took it out of that series' reach.
+__device__ __forceinline__ void bw_step64(double &x, double &f, double &nu, double &q, double z, const BW64 &c) {
+    const double t = __dmul_rn(c.ln_omr, __dmul_rn(__dsub_rn(1.0, f), rcp_fast(f)));
+    const int ie = exp_index(t), in_ = nu_index(nu);
+    if (!((unsigned)ie < (unsigned)BW_EXP && (unsigned)in_ < (unsigned)BW_NU)) {
+        const BWState s = bw_step64_any({x, f, nu, q}, z, c.dt, c.kappa, c.y, c.dt_itau, c.ialpha, c.irho, c.log2_omr);
+        x = s.x; f = s.f; nu = s.nu; q = s.q;
+        return;
+    }
+    const double2 ct = __ldg(reinterpret_cast<const double2 *>(c.tab) + in_);
+    double s = fma(-c.kappa, x, z);
+    s = fma(-c.y, __dsub_rn(f, 1.0), s);
+    x = fma(c.dt, s, x);
+    const double tf = fma(c.dt, x, f);
+    const double e = __dmul_rn(__ldg(c.tab + 2 * BW_NU + ie), exp_tiny(fma((double)(BW_EXP0 - ie), 0.125, t)));
+    double p = c.binom[BINOM_TERMS], d = fma(nu, ct.x, -1.0);
+#pragma unroll
+    for (int k = BINOM_TERMS - 1; k >= 0; --k) p = fma(p, d, c.binom[k]);
+    nu = fma(c.dt_itau, __dsub_rn(f, __dmul_rn(ct.y, p)), nu);
+    p = c.binom[BINOM_TERMS];
+    d = fma(nu, ct.x, -1.0);
+#pragma unroll
+    for (int k = BINOM_TERMS - 1; k >= 0; --k) p = fma(p, d, c.binom[k]);
+    p = __dmul_rn(ct.y, p);
+    if (!bw_in_reach(d)) p = bw_pow_any(nu, c.ialpha);
+    const double in = __dmul_rn(__dmul_rn(f, __dsub_rn(1.0, __dmul_rn(c.omr, e))), c.irho);
+    const double out = __dmul_rn(__dmul_rn(p, q), rcp_fast(nu));
+    q = fma(c.dt_itau, __dsub_rn(in, out), q);
+    f = tf;
+}
+__device__ __noinline__ BWState bw_step64_out(BWState s, double z, const BW64 *c) {
+    bw_step64(s.x, s.f, s.nu, s.q, z, *c);
+    return s;
+}
+
+// The step of N items, the operations of bw_step64 and so its bits, whatever the other
+// items are.  Where all are in the range that no step leaves the reach of its centre's
+// series from (|f - nu^(1/alpha)| dt/tau <= 0.0105 c: 0 < f <= 2^reach nu, compared by their
+// high words, and nu's centre below nu_end, see fill_bwf) there is no branch, so the items' chains of dependent FP64
+// operations overlap: with the range tests inside, two items took 2,700 cycles one after
+// the other in the tile kernel.  (Testing the reach itself, or selecting per item inside
+// one straight-line form, cost 2-5 % of the tile kernels' time.)
 template <int N>
 __device__ __forceinline__ void bw_step64_n(double (&x)[N], double (&f)[N], double (&nu)[N], double (&q)[N],
                                             const double (&z)[N], const BW64 &c) {
     double tf[N], t[N], p[N], r[N];
     int in_[N], ie[N];
-    bool in_range = c.dt_itau <= 0.002;   // a step then moves nu too little to leave its centre's series
+    bool in_range = true;
 #pragma unroll
     for (int u = 0; u < N; ++u) {
         t[u] = __dmul_rn(c.ln_omr, __dmul_rn(__dsub_rn(1.0, f[u]), rcp_fast(f[u])));
         ie[u] = exp_index(t[u]);
         in_[u] = nu_index(nu[u]);
-        in_range = in_range && (unsigned)ie[u] < (unsigned)BW_EXP && (unsigned)in_[u] < (unsigned)BW_NU;
+        in_range = in_range && (unsigned)ie[u] < (unsigned)BW_EXP && (unsigned)in_[u] < (unsigned)c.nu_end &&
+                   (unsigned)__double2hiint(f[u]) <= (unsigned)(__double2hiint(nu[u]) + c.reach);
     }
     if (!in_range) {
 #pragma unroll
-        for (int u = 0; u < N; ++u) bw_step64(x[u], f[u], nu[u], q[u], z[u], c);
+        for (int u = 0; u < N; ++u) {
+            const BWState s = bw_step64_out({x[u], f[u], nu[u], q[u]}, z[u], &c);
+            x[u] = s.x; f[u] = s.f; nu[u] = s.nu; q[u] = s.q;
+        }
         return;
     }
     double2 ct[N];
