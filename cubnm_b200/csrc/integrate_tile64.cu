@@ -8,11 +8,11 @@
 // 1,264 cycles per simulation with the SM full, of which the FP64 pipe (64 lanes an SM)
 // needs about 370.  Two forms replace it:
 //
-//  * k_one64, batches of up to four simulations per SM: one CTA per simulation.  The n x n
-//    product with x is spread over 4 lanes per node: a group of 16 lanes holds four rows
-//    of SC^T, each lane the sources k = lane mod 16, in registers; partial sums meet in a
-//    transposing butterfly (5 shuffles) and the update runs on one thread per node.  Bound
-//    by latency: product, two barriers, update chain.
+//  * k_one64, small batches: one CTA per simulation.  The n x n product with x is spread
+//    over the lanes: a group of eight holds four rows of SC^T, each lane one chain of the
+//    sources, in registers; partial sums meet in a transposing butterfly (4 shuffles) and
+//    the update runs on one thread per node.  Bound by latency: product, two barriers,
+//    update chain.
 //  * k_tile64, larger batches: eight simulations sharing an SC per CTA, the product as
 //    mma.sync m8n8k4 (FP64), SC^T fragments in registers, so that a weight read serves
 //    eight simulations and the sums need no shuffles.  DMMA runs at the FP64 pipe's rate
@@ -21,8 +21,17 @@
 //    simulation and step at 100 nodes, update about 180).  The Balloon-Windkessel model
 //    of a tile runs in up to four more warps, a millisecond behind.
 //
+// Both form a sum in one order, so that a simulation has the same bits in any batch: chain
+// (h, e), h < 4, e < 2, runs over sources 8 c + 2 t + e, c = h, h + 4, .., t = 0 .. 3, by
+// fused multiply-adds from zero (m8n8k4 adds its four products one after the other, rounding
+// each: equal to the chain of fma in all of 65,536 random sums); then e = 0 and e = 1 each
+// ((h0 + h2) + (h1 + h3)), then both.  Measured against two chains of free order: tiles
+// 1-5 % slower (rWW 100 nodes, 1,184 simulations, 21.9 -> 22.6 ms per simulated second), one
+// simulation at 100 nodes 8.2 -> 7.5 ms (four rows a group of eight lanes instead of two a
+// group of sixteen halve the loads of x; rWW 68 nodes 6.4 -> 6.5).
+//
 // Noise rows are copied to shared memory a chunk of steps ahead.  The sums are formed in
-// another order than the reference's, with fused multiply-adds.
+// another order than the reference's, and multiply-adds are fused, in the update too.
 #include <algorithm>
 #include <cstdint>
 #include "engine.h"
@@ -90,31 +99,42 @@ __device__ __forceinline__ void states_mean(const IntegrateArgs &a, int sim, int
     }
 }
 
+// Place of source k in k_one64's x: a lane reads two of its chain's sources in 16 bytes, the
+// eight lanes of a group 128 in a row.
+__device__ __forceinline__ int one_pos(int k) {
+    const int t = (k >> 1) & 3, l = ((k >> 3) & 3) * 2 + (k & 1);
+    return ((k >> 5) * 4 + (t & 2)) * 8 + 2 * l + (t & 1);
+}
+
 __device__ __forceinline__ double bold_of(const IntegrateArgs &a, double q, double nu) {  // bnm.cpp:316-335
     return a.bw.V_0 * (a.bw.k1 * (1 - q) + a.bw.k2 * (1 - q / nu) + a.bw.k3 * (1 - nu));
 }
 
 // ---------------------------------------------------------------- one simulation per CTA
-// KPL: compiled sources per lane (16 KPL >= n).
-template <class M, int KPL>
-__global__ void __launch_bounds__(KPL * 64) k_one64(const __grid_constant__ IntegrateArgs a) {
+__host__ __device__ constexpr bool one_par_smem(int nc) { return nc == 3; }   // parameters too
+// NC: compiled count of 32-source blocks (32 NC >= n).  The Balloon-Windkessel state,
+// touched once a millisecond, is in shared memory: the weights take 32 NC registers.
+template <class M, int NC>
+__global__ void __launch_bounds__(NC * 64) k_one64(const __grid_constant__ IntegrateArgs a) {
     constexpr int NN = M::NN;
+    constexpr bool PAR_SMEM = one_par_smem(NC);
     extern __shared__ __align__(16) double sh[];
-    const int n = a.nodes, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = lane & 15, nwarps = blockDim.x >> 5;
+    const int n = a.nodes, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = lane & 7, nwarps = blockDim.x >> 5;
     const int chunk = min(a.inner_it, NOISE_CHUNK);
-    double *x = sh, *in_s = x + 16 * KPL, *noise_s = in_s + 16 * KPL;   // [16 KPL], [16 KPL], [2][chunk][n][NN]
-    const int row0 = warp * 8 + (lane >> 4) * 4;                        // the four rows of this half-warp
-    const int my_row = row0 + (l >> 3) * 2 + ((l >> 2) & 1);            // the row whose sum this lane ends with
+    double *x = sh, *in_s = x + 32 * NC, *bws = in_s + 32 * NC, *par = bws + 128 * NC;   // [32 NC], [32 NC], [4][32 NC]
+    double *noise_s = par + (PAR_SMEM ? (M::NR + M::NG) * 32 * NC : 0);   // parameters [NR + NG][32 NC]; noise [2][chunk][n][NN]
+    const int row0 = warp * 16 + (lane >> 3) * 4;                     // the four rows of this group of eight lanes
+    const int my_row = row0 + (l >> 1);                               // the row whose sum this lane ends with
     const int j = tid;
     const bool act = j < n;
     for (int sim = blockIdx.x; sim < a.n_sims; sim += gridDim.x) {
         const double *SC = a.sc + (size_t)a.sc_idx[sim] * n * n;
-        double w[4][KPL];
+        double w[4][4 * NC];   // chain l: sources 32 b + 8 (l / 2) + 2 t + l % 2
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int i = 0; i < KPL; ++i) {
-                const int k = l + 16 * i;
+            for (int i = 0; i < 4 * NC; ++i) {
+                const int k = (i >> 2) * 32 + (l >> 1) * 8 + 2 * (i & 3) + (l & 1);
                 w[r][i] = row0 + r < n && k < n ? SC[(size_t)k * n + row0 + r] : 0.0;
             }
         double g[M::NG], iv[M::NI], r[M::NR], s[M::NS];
@@ -128,9 +148,20 @@ __global__ void __launch_bounds__(KPL * 64) k_one64(const __grid_constant__ Inte
 #pragma unroll
         for (int i = 0; i < M::NS; ++i) s[i] = 0.0;
         M::init(s, iv, g, r);
-        double bx = 0.0, bf = 1.0, bnu = 1.0, bq = 1.0;
-        double *bold = a.bold + (size_t)sim * a.bold_len * n;
-        if (tid < 16 * KPL) x[tid] = act ? s[M::CONN] : 0.0;
+        if (PAR_SMEM && act) {
+#pragma unroll
+            for (int i = 0; i < M::NR; ++i) par[i * 32 * NC + j] = r[i];
+#pragma unroll
+            for (int i = 0; i < M::NG; ++i) par[(M::NR + i) * 32 * NC + j] = g[i];
+        }
+        double *const b = bws + j;   // x, f, nu, q at stride 32 NC
+        if (act) {
+            b[0] = 0.0;
+            b[32 * NC] = b[64 * NC] = b[96 * NC] = 1.0;
+        }
+        for (int k = tid; k < 32 * NC; k += blockDim.x) x[k] = 0.0;   // padding
+        __syncthreads();
+        if (act) x[one_pos(j)] = s[M::CONN];
         stage_noise<NN>(a, 0, 0, chunk, noise_s, nwarps);
         cp_commit();
         cp_wait_all();
@@ -147,38 +178,57 @@ __global__ void __launch_bounds__(KPL * 64) k_one64(const __grid_constant__ Inte
                 for (int inner = i0; inner < i1; ++inner) {
                     double v[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-                    for (int i = 0; i < KPL; ++i) {
-                        const double xk = x[l + 16 * i];
+                    for (int i = 0; i < 4 * NC; i += 2) {
+                        const double2 xk = *reinterpret_cast<const double2 *>(x + i * 8 + 2 * l);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) v[q] = fma(w[q][i], xk, v[q]);
+                        for (int q = 0; q < 4; ++q) v[q] = fma(w[q][i + 1], xk.y, fma(w[q][i], xk.x, v[q]));
                     }
                     // transposing butterfly: lanes keep rows {0,1} / {2,3}, then one row, then its sum
-                    const bool up = l & 8, odd = l & 4;
-                    double s0 = up ? v[0] : v[2], s1 = up ? v[1] : v[3];
+                    const bool up = l & 4, odd = l & 2;
                     double m0 = up ? v[2] : v[0], m1 = up ? v[3] : v[1];
-                    m0 += __shfl_xor_sync(0xffffffffu, s0, 8);
-                    m1 += __shfl_xor_sync(0xffffffffu, s1, 8);
-                    s0 = odd ? m0 : m1;
-                    m0 = odd ? m1 : m0;
-                    m0 += __shfl_xor_sync(0xffffffffu, s0, 4);
-                    m0 += __shfl_xor_sync(0xffffffffu, m0, 2);
-                    m0 += __shfl_xor_sync(0xffffffffu, m0, 1);
-                    if ((l & 3) == 0) in_s[my_row] = m0;
+                    m0 += __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 4);
+                    m1 += __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 4);
+                    double m = odd ? m1 : m0;
+                    m += __shfl_xor_sync(0xffffffffu, odd ? m0 : m1, 2);
+                    m += __shfl_xor_sync(0xffffffffu, m, 1);
+                    if ((l & 1) == 0) in_s[my_row] = m;
                     __syncthreads();
                     if (act) {
                         const double *z = noise_s + ((size_t)(nbuf * chunk + inner - i0) * n + j) * NN;
+                        if constexpr (PAR_SMEM) {
+#pragma unroll
+                            for (int i = 0; i < M::NR; ++i) r[i] = par[i * 32 * NC + j];
+#pragma unroll
+                            for (int i = 0; i < M::NG; ++i) g[i] = par[(M::NR + i) * 32 * NC + j];
+                        }
                         M::step(s, iv, g, r, in_s[j], z[0], NN > 1 ? z[NN - 1] : 0.0, a.K);
-                        x[j] = s[M::CONN];
+                        x[one_pos(j)] = s[M::CONN];
+                    } else {   // assigned on every path, outputs of a step hold no register during the product
+#pragma unroll
+                        for (int i = 0; i < M::NS; ++i) s[i] = 0.0;
+#pragma unroll
+                        for (int i = 0; i < M::NI; ++i) iv[i] = 0.0;
+                        if constexpr (PAR_SMEM) {
+#pragma unroll
+                            for (int i = 0; i < M::NR; ++i) r[i] = 0.0;
+#pragma unroll
+                            for (int i = 0; i < M::NG; ++i) g[i] = 0.0;
+                        }
                     }
                     if (inner == i1 - 1) cp_wait_all();   // the next chunk's noise, before the barrier
                     __syncthreads();
                 }
                 nbuf ^= 1;
             }
-            if (act) bw_step64(bx, bf, bnu, bq, s[M::BOLDV], a.bwf);
-            if (--to_tr == 0) {
+            const bool tr = --to_tr == 0;
+            if (act) {
+                double bx = b[0], bf = b[32 * NC], bnu = b[64 * NC], bq = b[96 * NC];
+                bw_step64(bx, bf, bnu, bq, s[M::BOLDV], a.bwf);
+                b[0] = bx; b[32 * NC] = bf; b[64 * NC] = bnu; b[96 * NC] = bq;
+                if (tr && bold_i < a.bold_len) a.bold[((size_t)sim * a.bold_len + bold_i) * n + j] = bold_of(a, bq, bnu);
+            }
+            if (tr) {
                 to_tr = a.bold_tr_iters;
-                if (act && bold_i < a.bold_len) bold[(size_t)bold_i * n + j] = bold_of(a, bq, bnu);
                 ++bold_i;   // a sample past bold_len has no slot
             }
             if (--to_sample == 0) {
@@ -218,6 +268,7 @@ __host__ __device__ constexpr int min_ctas(int ks) { return ks <= 4 ? 2 : 1; }
 
 // The Balloon-Windkessel warps: for every tile and millisecond, wait for the inputs of the
 // 8 n items (item s n + j), step them two at a time, write BOLD at TR.
+template <bool CALL>
 __device__ __forceinline__ void bw_items(const IntegrateArgs &a, const int *td, double *b, const double *z, int tid, int nthr,
                                          bool tr, int bold_i) {
     const int n = a.nodes, items = TS * n;
@@ -229,7 +280,7 @@ __device__ __forceinline__ void bw_items(const IntegrateArgs &a, const int *td, 
             x[u] = b[at[u]]; f[u] = b[items + at[u]]; nu[u] = b[2 * items + at[u]]; q[u] = b[3 * items + at[u]];
             zz[u] = z[at[u]];
         }
-        bw_step64_n<2>(x, f, nu, q, zz, a.bwf);
+        bw_step64_n<2, CALL>(x, f, nu, q, zz, a.bwf);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             b[at[u]] = x[u]; b[items + at[u]] = f[u]; b[2 * items + at[u]] = nu[u]; b[3 * items + at[u]] = q[u];
@@ -240,6 +291,7 @@ __device__ __forceinline__ void bw_items(const IntegrateArgs &a, const int *td, 
         }
     }
 }
+template <bool CALL>
 __device__ __forceinline__ void bw_role(const IntegrateArgs &a, double *b, const double *zs, int tid, int nthr) {
     const int items = TS * a.nodes;
     for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
@@ -252,7 +304,7 @@ __device__ __forceinline__ void bw_role(const IntegrateArgs &a, double *b, const
         for (int bw_i = 0; bw_i < a.bw_it; ++bw_i) {
             const bool tr = --to_tr == 0;
             bar_sync(2, blockDim.x);
-            bw_items(a, td, b, zs + (bw_i & 1) * items, tid, nthr, tr, bold_i);
+            bw_items<CALL>(a, td, b, zs + (bw_i & 1) * items, tid, nthr, tr, bold_i);
             if (tr) {
                 to_tr = a.bold_tr_iters;
                 ++bold_i;
@@ -266,6 +318,7 @@ __device__ __forceinline__ void bw_role(const IntegrateArgs &a, double *b, const
 template <class M, int KS>
 __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_tile64(const __grid_constant__ IntegrateArgs a) {
     constexpr int NN = M::NN;
+    constexpr bool BW_CALL = KS >= 13;   // see bw_step64_n
     extern __shared__ __align__(16) unsigned char smem[];
     const int n = a.nodes, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -277,7 +330,7 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_tile
     const int items = TS * n, node_threads = L.mt * 32;
     const bool bw_here = bw_warps(L.mt) == 0;   // 16 node warps: they do the Balloon-Windkessel work themselves
     if (warp >= L.mt) {
-        bw_role(a, bws, zs, tid - node_threads, nthr - node_threads);
+        bw_role<BW_CALL>(a, bws, zs, tid - node_threads, nthr - node_threads);
         return;
     }
     const int j = warp * 8 + g;                 // this lane's node; simulations 2t, 2t + 1 of the tile
@@ -341,20 +394,39 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_tile
                 cp_commit();
                 const int i1 = min(i0 + chunk, a.inner_it);
                 for (int inner = i0; inner < i1; ++inner) {
-                    double d[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
                     const double *xr = xc + g * L.rs + 2 * t;
+                    auto chain = [&](int h, double (&d)[2][2]) {   // 8-source tiles h, h + 4, ..
+                        d[0][0] = d[0][1] = d[1][0] = d[1][1] = 0.0;
 #pragma unroll
-                    for (int c = 0; c < KS; ++c) {
-                        if (c < L.mt) {
-                            const double2 b = *reinterpret_cast<const double2 *>(xr + 8 * c);
-                            mma_f64(d[0], w[c][0], b.x);
-                            mma_f64(d[1], w[c][1], b.y);
-                        }
+                        for (int c = h; c < KS; c += 4)
+                            if (c < L.mt) {
+                                const double2 b = *reinterpret_cast<const double2 *>(xr + 8 * c);
+                                mma_f64(d[0], w[c][0], b.x);
+                                mma_f64(d[1], w[c][1], b.y);
+                            }
+                    };
+                    double in2[2], d0[2][2], d1[2][2];
+                    {
+                        double d2[2][2];
+                        chain(0, d0);
+                        chain(2, d2);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+#pragma unroll
+                            for (int u = 0; u < 2; ++u) d0[e][u] += d2[e][u];
+                        chain(1, d1);
+                        chain(3, d2);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+#pragma unroll
+                            for (int u = 0; u < 2; ++u) d0[e][u] += d1[e][u] + d2[e][u];
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) in2[u] = d0[0][u] + d0[1][u];
                     }
                     const double *z = noise_s + ((size_t)(nbuf * chunk + inner - i0) * n + jn) * NN;
                     const double n0 = z[0], n1 = NN > 1 ? z[NN - 1] : 0.0;
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) M::step(s[u], iv[u], gl[u], r[u], d[0][u] + d[1][u], n0, n1, a.K);
+                    for (int u = 0; u < 2; ++u) M::step(s[u], iv[u], gl[u], r[u], in2[u], n0, n1, a.K);
                     write_x(xn);
                     if (inner == i1 - 1) cp_wait_all();   // the next chunk's noise, before the barrier
                     bar_sync(1, node_threads);
@@ -372,7 +444,7 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_tile
             }
             bar_sync(2, nthr);
             const bool tr = --to_tr == 0;
-            if (bw_here) bw_items(a, td, bws, z, tid, nthr, tr, bold_i);
+            if (bw_here) bw_items<BW_CALL>(a, td, bws, z, tid, nthr, tr, bold_i);
             if (tr) {
                 to_tr = a.bold_tr_iters;
                 ++bold_i;
@@ -395,48 +467,73 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_tile
     }
 }
 
+// CTAs an SM holds.
 template <class K>
-cudaError_t launch(K kernel, const IntegrateArgs &a, int items, int threads, size_t smem, cudaStream_t st) {
-    cudaError_t e = allow_dynamic_smem(kernel);
-    int dev = 0, sms = 0, occ = 0;
+cudaError_t occupancy(K kernel, int threads, size_t smem, int *occ) {
+    const cudaError_t e = allow_dynamic_smem(kernel);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kernel, threads, smem);
+}
+int sm_count() {
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
+    return sms;
+}
+
+// A kernel's instance for a run: launched over `items`, or with occ set, only asked for its occupancy.
+template <class K>
+cudaError_t use(K kernel, const IntegrateArgs &a, int items, int threads, size_t smem, cudaStream_t st, int *occ) {
+    int fits = 0;
+    const cudaError_t e = occupancy(kernel, threads, smem, &fits);
     if (e != cudaSuccess) return e;
-    if (occ < 1) return cudaErrorInvalidConfiguration;
-    kernel<<<std::min(items, occ * sms), threads, smem, st>>>(a);
+    if (fits < 1) return cudaErrorInvalidConfiguration;
+    if (occ) {
+        *occ = fits;
+        return cudaSuccess;
+    }
+    kernel<<<std::min(items, fits * sm_count()), threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <class M, int KPL>
-cudaError_t launch_one(const IntegrateArgs &a, cudaStream_t st) {
+template <class M, int NC>
+cudaError_t use_one(const IntegrateArgs &a, cudaStream_t st, int *occ) {
     const int chunk = std::min(a.inner_it, NOISE_CHUNK);
-    const size_t smem = 8 * ((size_t)32 * KPL + (size_t)2 * chunk * a.nodes * M::NN);
-    return launch(k_one64<M, KPL>, a, a.n_sims, ((a.nodes + 7) / 8) * 32, smem, st);
+    const size_t smem = 8 * ((size_t)(192 + (one_par_smem(NC) ? 32 * (M::NR + M::NG) : 0)) * NC + (size_t)2 * chunk * a.nodes * M::NN);
+    return use(k_one64<M, NC>, a, a.n_sims, ((a.nodes + 15) / 16) * 32, smem, st, occ);
 }
 template <class M, int KS>
-cudaError_t launch_tile(const IntegrateArgs &a, cudaStream_t st) {
+cudaError_t use_tile(const IntegrateArgs &a, cudaStream_t st, int *occ) {
     const Layout L = layout(a.nodes, M::NN, std::min(a.inner_it, NOISE_CHUNK));
-    return launch(k_tile64<M, KS>, a, a.n_tiles, (L.mt + bw_warps(L.mt)) * 32, L.bytes, st);
+    return use(k_tile64<M, KS>, a, a.n_tiles, (L.mt + bw_warps(L.mt)) * 32, L.bytes, st, occ);
 }
 
 // Compiled extents; a run takes the least that holds its nodes.
 template <class M>
-cudaError_t launch_model(const IntegrateArgs &a, cudaStream_t st) {
-    if (!a.tiles) {
-        const int kpl = (a.nodes + 15) / 16;
-        if (kpl <= 2) return launch_one<M, 2>(a, st);
-        if (kpl <= 4) return launch_one<M, 4>(a, st);
-        if (kpl <= 5) return launch_one<M, 5>(a, st);
-        if (kpl <= 7) return launch_one<M, 7>(a, st);
-        return launch_one<M, 8>(a, st);
+cudaError_t use_model(const IntegrateArgs &a, bool tiles, cudaStream_t st, int *occ) {
+    if (!tiles) {
+        const int nc = (a.nodes + 31) / 32;
+        if (nc <= 1) return use_one<M, 1>(a, st, occ);
+        if (nc <= 2) return use_one<M, 2>(a, st, occ);
+        if (nc <= 3) return use_one<M, 3>(a, st, occ);
+        return use_one<M, 4>(a, st, occ);
     }
     const int mt = (a.nodes + 7) / 8;
-    if (mt <= 4) return launch_tile<M, 4>(a, st);
-    if (mt <= 8) return launch_tile<M, 8>(a, st);
-    if (mt <= 11) return launch_tile<M, 11>(a, st);
-    if (mt <= 13) return launch_tile<M, 13>(a, st);
-    return launch_tile<M, 16>(a, st);
+    if (mt <= 4) return use_tile<M, 4>(a, st, occ);
+    if (mt <= 8) return use_tile<M, 8>(a, st, occ);
+    if (mt <= 11) return use_tile<M, 11>(a, st, occ);
+    if (mt <= 13) return use_tile<M, 13>(a, st, occ);
+    return use_tile<M, 16>(a, st, occ);
+}
+
+cudaError_t use_any(int model, const IntegrateArgs &a, bool tiles, cudaStream_t st, int *occ) {
+    switch (model) {
+        case MODEL_RWW: return use_model<RWWm<double>>(a, tiles, st, occ);
+        case MODEL_WC: return use_model<WCm<double>>(a, tiles, st, occ);
+        case MODEL_JR: return use_model<JRm<double>>(a, tiles, st, occ);
+        case MODEL_RWWEX: return use_model<RWWExm<double>>(a, tiles, st, occ);
+        default: break;
+    }
+    return cudaErrorNotSupported;
 }
 
 }  // namespace
@@ -448,14 +545,7 @@ bool tile64_supported(int model, int nodes) {
 }
 
 cudaError_t launch_integrate_tile64(int model, const IntegrateArgs &a, cudaStream_t st) {
-    switch (model) {
-        case MODEL_RWW: return launch_model<RWWm<double>>(a, st);
-        case MODEL_WC: return launch_model<WCm<double>>(a, st);
-        case MODEL_JR: return launch_model<JRm<double>>(a, st);
-        case MODEL_RWWEX: return launch_model<RWWExm<double>>(a, st);
-        default: break;
-    }
-    return cudaErrorNotSupported;
+    return use_any(model, a, a.tiles != nullptr, st, nullptr);
 }
 
 }  // namespace cbnm

@@ -1164,11 +1164,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     }
     // FP64 without delays or numerical FIC, up to 128 nodes: the register-resident forms
     // (integrate_tile64.cu) unless a coupling form of the per-simulation kernel is forced.
-    // Up to four simulations per SM run one per CTA, more in tiles of eight: at 100 nodes a
-    // step of a tile takes about four times a single simulation's, and N / 8 tiles must
-    // fill the SMs.
     const bool t64 = !c.fp32 && !has_delay && !num_fic && tile64_supported(md.id, n) && !std::getenv("CBNM_COUPLING");
-    const bool t64_tiles = t64 && N > 4 * sm_count();
+    bool t64_tiles = false;
     if (!use_tc && !delay_blocks && !t64) {
         // Sparse coupling for the per-simulation kernels (ELLPACK by target node):
         // used when the densest column of every SC holds at most half the nodes
@@ -1379,7 +1376,9 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         CK(launch_integrate_simt32(md.id, ia, S.st));
         ++launches;
     } else if (t64) {
-        if (t64_tiles) put_tiles(make_tiles(FP64_TILE));
+        const std::vector<int> tiles = make_tiles(FP64_TILE);
+        t64_tiles = N > 4 * sm_count();
+        if (t64_tiles) put_tiles(tiles);
         CK(cudaEventRecord(S.ev[1], S.st));
         CK(launch_integrate_tile64(md.id, ia, S.st));
         ++launches;

@@ -474,7 +474,11 @@ __device__ __noinline__ BWState bw_step64_out(BWState s, double z, const BW64 *c
 // operations overlap: with the range tests inside, two items took 2,700 cycles one after
 // the other in the tile kernel.  (Testing the reach itself, or selecting per item inside
 // one straight-line form, cost 2-5 % of the tile kernels' time.)
-template <int N>
+// CALL: items out of that range go through a function, else through code in line.  The call
+// makes FP64 tiles of up to 88 nodes spill (rWW, 32 nodes, 10.6 against 6.2 ms per simulated
+// second and 1,184 simulations), the code in line larger ones (JR, 128 nodes, 41.7 against
+// 36.2) and the FP32 tiles.
+template <int N, bool CALL = true>
 __device__ __forceinline__ void bw_step64_n(double (&x)[N], double (&f)[N], double (&nu)[N], double (&q)[N],
                                             const double (&z)[N], const BW64 &c) {
     double tf[N], t[N], p[N], r[N];
@@ -489,10 +493,24 @@ __device__ __forceinline__ void bw_step64_n(double (&x)[N], double (&f)[N], doub
                    (unsigned)__double2hiint(f[u]) <= (unsigned)(__double2hiint(nu[u]) + c.reach);
     }
     if (!in_range) {
+        if constexpr (CALL) {
 #pragma unroll
-        for (int u = 0; u < N; ++u) {
-            const BWState s = bw_step64_out({x[u], f[u], nu[u], q[u]}, z[u], &c);
-            x[u] = s.x; f[u] = s.f; nu[u] = s.nu; q[u] = s.q;
+            for (int u = 0; u < N; ++u) {
+                const BWState s = bw_step64_out({x[u], f[u], nu[u], q[u]}, z[u], &c);
+                x[u] = s.x; f[u] = s.f; nu[u] = s.nu; q[u] = s.q;
+            }
+        } else {
+            static_assert(N == 2, "one copy of the code, the items swapped between its two turns");
+            auto swap = [](double (&v)[N]) {
+                const double w = v[0];
+                v[0] = v[1];
+                v[1] = w;
+            };
+#pragma unroll 1
+            for (int u = 0; u < 2; ++u) {
+                bw_step64(x[0], f[0], nu[0], q[0], u ? z[1] : z[0], c);
+                swap(x); swap(f); swap(nu); swap(q);
+            }
         }
         return;
     }
