@@ -206,6 +206,7 @@ cudaError_t launch_integrate_mma(int model, const IntegrateArgs &a, cudaStream_t
 // SC where a.tiles is set (laid out as above), else one simulation per CTA.
 constexpr int FP64_TILE = 8;
 bool tile64_supported(int model, int nodes);
+cudaError_t tile64_choose(int model, const IntegrateArgs &a, int n_tiles, bool *tiles);   // which of the two is faster
 cudaError_t launch_integrate_tile64(int model, const IntegrateArgs &a, cudaStream_t st);
 void fill_k32(int model, const ModelK &K, float *k32);   // the model's FP32 constants
 // Conduction delays, blocks of 32 steps (integrate_delay.cuh).

@@ -536,7 +536,32 @@ cudaError_t use_any(int model, const IntegrateArgs &a, bool tiles, cudaStream_t 
     return cudaErrorNotSupported;
 }
 
+// Time of `items` CTAs of which an SM holds occ at once, in units of one alone on its SM;
+// each further one on an SM adds `share` of that.
+double waves(int items, int occ, double share) {
+    const int sms = sm_count(), load = (items + sms - 1) / sms;   // CTAs of the fullest SM
+    const int full = load / occ, rest = load % occ;
+    return full * (1.0 + share * (occ - 1)) + (rest ? 1.0 + share * (rest - 1) : 0.0);
+}
+
 }  // namespace
+
+// Whether n_tiles tiles of eight are faster than n_sims CTAs of one simulation: by the
+// waves that either form takes on this GPU.  A tile's step takes n / 34 of a single
+// simulation's, at least 1.25 (ms per simulated second alone on an SM, one / tile: rWW 32
+// nodes 5.2 / 6.3, 64 nodes 5.5 / 9.8, 68 nodes 6.5 / 14.4, 100 nodes 7.5 / 22.6, 128 nodes
+// 7.5 / 27.6; WC 100 nodes 7.0 / 22.6, JR 9.7 / 30.7, rWWEx 6.3 / 18.3), a second CTA on an
+// SM costs a fifth more (rWW 68 nodes 6.5 -> 7.8).  So 444 simulations of 100 nodes on 148
+// SMs take 22.6 ms in either form, 450 take 22.6 in tiles and 30.1 one by one, and 600 with
+// an SC each (600 tiles of one live column) 113 in tiles and 37.7 one by one.
+cudaError_t tile64_choose(int model, const IntegrateArgs &a, int n_tiles, bool *tiles) {
+    int occ1 = 0, occ8 = 0;
+    cudaError_t e = use_any(model, a, false, nullptr, &occ1);
+    if (e == cudaSuccess) e = use_any(model, a, true, nullptr, &occ8);
+    if (e != cudaSuccess) return e;
+    *tiles = std::max(1.25, a.nodes / 34.0) * waves(n_tiles, occ8, 0.3) < waves(a.n_sims, occ1, 0.2);
+    return cudaSuccess;
+}
 
 // Without delays and numerical FIC (whose restarts are per simulation), up to 128 nodes.
 bool tile64_supported(int model, int nodes) {

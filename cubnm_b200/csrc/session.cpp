@@ -1377,7 +1377,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         ++launches;
     } else if (t64) {
         const std::vector<int> tiles = make_tiles(FP64_TILE);
-        t64_tiles = N > 4 * sm_count();
+        CK(tile64_choose(md.id, ia, ia.n_tiles, &t64_tiles));
         if (t64_tiles) put_tiles(tiles);
         CK(cudaEventRecord(S.ev[1], S.st));
         CK(launch_integrate_tile64(md.id, ia, S.st));

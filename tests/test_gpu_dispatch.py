@@ -8,11 +8,14 @@ from cubnm_b200 import core
 pytestmark = pytest.mark.gpu
 
 
-def _run(model, nodes, N, precision, velocity=0.0, density=0.3, **config):
+def _run(model, nodes, N, precision, velocity=0.0, density=0.3, scs=1, **config):
     a = list(cases.synthetic_args(model, N=N, nodes=nodes, duration_s=1, seed=nodes, density=density,
                                   G=np.linspace(0.2, 1.2, N), bold_remove_s=0, do_fcd=False, precision=precision))
     a[7] = dict(a[7], do_fc="0", noise_time_steps="100", **config)
     a[16], a[17], a[18] = 100, 100, 100
+    if scs > 1:
+        a[1] = np.stack([cases.synthetic_sc(nodes, density, s).reshape(-1) for s in range(scs)])
+        a[2] = (np.arange(N) % scs).astype(np.intc)
     if velocity:
         a[3] = np.ascontiguousarray(cases.synthetic_lengths(nodes, nodes).ravel())
         a[6] = np.full(N, velocity)
@@ -28,6 +31,15 @@ def _run(model, nodes, N, precision, velocity=0.0, density=0.3, **config):
     ("JR", 200, 9, "fp32", "k_integrate_mma"), ("rWW", 225, 9, "fp32", "k_integrate_sim")])
 def test_without_delays(model, nodes, N, precision, kernel):
     assert _run(model, nodes, N, precision) == kernel
+
+
+@pytest.mark.parametrize("nodes,N,scs,kernel", [
+    (100, 148, 1, "k_one64"), (100, 450, 1, "k_tile64"), (100, 592, 1, "k_tile64"), (68, 450, 1, "k_tile64"),
+    (100, 600, 75, "k_tile64"), (100, 600, 600, "k_one64"), (32, 1184, 1, "k_tile64"), (32, 1000, 1000, "k_one64")])
+def test_fp64_form_by_waves(nodes, N, scs, kernel):
+    """Tiles of eight where they finish first on 148 SMs: not for few simulations, nor where
+    each has an SC of its own and a tile one live column."""
+    assert _run("rWW", nodes, N, "fp64", scs=scs) == kernel
 
 
 @pytest.mark.parametrize("model,nodes,precision,density,kernel", [
