@@ -15,11 +15,12 @@
 //    96 nodes lo in shared memory); a step loads the eight simulations' x as B
 //    fragments (one 16-byte load per 16 sources brings hi and lo) and issues the
 //    products hi hi, hi lo, lo hi.  FP16, with each row of SC^T scaled by a power of two
-//    and lo by 2^11, holds 22 bits (x is at most 1 in all four models), so that the sums
-//    are as exact as FP32 ones: BOLD of 40 rWW simulations against FP64, relative, 200
-//    nodes, 2.8e-8 with FP32 sums, 3.2e-8 so; 100 nodes 4.3e-8, 1.2e-7 in BF16 halves
-//    (the tcgen05 form).  The tensor pipe truncates where it accumulates:
-//    hi hi products chained over the K steps gave 9.1e-8, so the FP32 pipe adds them;
+//    and lo by 2^11, holds 22 bits (x is at most 1 in all four models).  The tensor pipe
+//    truncates where it accumulates: hi hi products chained over the K steps gave three
+//    times the error in BOLD, so the FP32 pipe adds them, and above 128 nodes the mean of
+//    what is lost within one product is added back (HH_BIAS).  Errors against FP64 beside
+//    launch_integrate_mma; 100-node rWW 3.3e-8 relative in BOLD, 1.1e-7 in BF16 halves (the
+//    tcgen05 form);
 //  * the accumulator layout is the update's layout: lane (g, t) holds nodes g, g + 8 of
 //    the warp and simulations 2t, 2t + 1, state and parameters in registers, stepped as
 //    pairs in packed FP32x2.  K is ordered so that the two nodes of a lane are adjacent
@@ -36,7 +37,7 @@
 // mma.sync reaches a quarter of tcgen05's rate on sm_100a (measured 950 FP16 multiply-
 // adds a cycle and SM), but a tile's 147 products at 100 nodes are 316 cycles of it, in
 // the shadow of the other CTA's update.  Measured at 100 nodes: 1,492 cycles a step with
-// one CTA an SM (8 simulations), 2,262 with two (200 nodes, one: 3,612).  What bounds a step then: the phases of a
+// one CTA an SM (8 simulations), 2,262 with two (200 nodes, one: 3,930).  What bounds a step then: the phases of a
 // CTA's warps (product, MUFU, update) follow one another between its barriers, with two
 // CTAs to overlap; more do not fit the registers.
 #include <algorithm>
@@ -44,6 +45,7 @@
 #include <cstdint>
 #include <cstring>
 #include <cuda_fp16.h>
+#include <type_traits>
 #include "engine.h"
 #include "tc_common.cuh"
 
@@ -61,6 +63,12 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint4 &a, uint32_t 
 }
 // v = hi + lo / LO_SCALE to 22 bits for 2^-14 <= |v| < 2^15, to 2^-36 below.
 constexpr float LO_SCALE = 2048.0f;
+// Share of the hi hi sums added back above 128 nodes and for rWWEx above 80, 2^-25: the tensor pipe drops what is
+// below the last place of the largest of its 16 products, on average half a unit of that
+// place a product, always towards zero (mean of the relative error of sums of 16 positive
+// products, x in [0.05, 0.95]: -4.0e-8 with all weights nonzero, -1.5e-8 with a quarter of
+// them; 2^-25 is 2.98e-8).
+constexpr float HH_BIAS = 2.98023224e-8f;
 __device__ __forceinline__ void split_f16x2(float2 v, uint32_t &hi, uint32_t &lo) {
     const __half2 h = __float22half2_rn(v);
     const float2 hf = __half22float2(h);
@@ -83,6 +91,35 @@ __device__ __forceinline__ void cp_small(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// rWWEx with the FP32 update of the per-simulation kernels (models.cuh, rwwex.cpp:48-73),
+// a pair of simulations at a time.
+struct RWWExs32 {
+    using K = ModelKf;
+    static constexpr bool PAIR = true, ACC = true;
+    static constexpr int NP = 4, NS = 1, NN = 1, NOUT = 3, CV = 0, BV = 0;
+    __device__ static void params(float *p, double G, const double *r, const K &k) {   // w J_N, G J_N, I_0, sigma
+        p[0] = (float)r[0] * k.rwwex.J_N; p[1] = (float)G * k.rwwex.J_N; p[2] = (float)r[1]; p[3] = (float)r[2];
+    }
+    __device__ static void pair_params(float2 *) {}
+    __device__ static void init(float *s) { s[0] = 0.001f; }
+    __device__ static void step2(float2 *s, const float2 *p, float2 in, float n0, float, const K &k, float2 *o) {
+        const RWWExKt<float> &m = k.rwwex;
+        const float2 x = __fadd2_rn(__ffma2_rn(p[1], in, __fmul2_rn(p[0], s[0])), p[2]);
+        const float2 r = rate2_acc(__ffma2_rn(f2(m.a), x, f2(-m.b)), m.d, 1.0f / m.d);
+        float2 ds = __fmul2_rn(f2(m.dt_gamma), __fmul2_rn(__ffma2_rn(s[0], f2(-1.0f), f2(1.0f)), r));
+        ds = __ffma2_rn(f2(-m.dt_itau), s[0], ds);
+        ds = __ffma2_rn(f2(n0 * m.sqrt_dt), p[3], ds);
+        const float2 n = __fadd2_rn(s[0], ds);
+        s[0] = make_float2(__saturatef(n.x), __saturatef(n.y));
+        o[0] = x; o[1] = r; o[2] = s[0];
+    }
+};
+template <class M>
+__device__ __forceinline__ const typename M::K &model_consts(const IntegrateArgs &a) {
+    if constexpr (std::is_same<typename M::K, ModelKf>::value) return a.Kf;
+    else return *reinterpret_cast<const typename M::K *>(a.k32);
+}
 
 // Shared-memory layout, from the node count and the model's noise terms.
 struct Layout {
@@ -176,7 +213,7 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
     float *zs = reinterpret_cast<float *>(smem + L.z);
     const int items = TS * n, node_threads = L.mt * 32;
     uint4 *alo_s = reinterpret_cast<uint4 *>(smem + L.alo) + (size_t)warp * KS * 32 + lane;
-    const typename M::K &K = *reinterpret_cast<const typename M::K *>(a.k32);
+    const typename M::K &K = model_consts<M>(a);
     const size_t rstride = (size_t)a.n_sims * n;
     const size_t ext = a.states_ts ? (size_t)n * a.states_len : (size_t)n;
     const int node[2] = {warp * 16 + g, warp * 16 + g + 8};
@@ -318,7 +355,9 @@ __global__ void __launch_bounds__((KS + bw_warps(KS)) * 32, min_ctas(KS)) k_inte
                         }
                         float2 o[M::NOUT];
                         const float lo_unscale = unscale[u] * (1.0f / LO_SCALE);
-                        const float2 in = __ffma2_rn(make_float2(hl[2 * u] + lh[2 * u], hl[2 * u + 1] + lh[2 * u + 1]),
+                        float2 lo = make_float2(hl[2 * u] + lh[2 * u], hl[2 * u + 1] + lh[2 * u + 1]);
+                        if constexpr (KS > 8 || M::ACC) lo = __ffma2_rn(hh[u], make_float2(HH_BIAS * LO_SCALE, HH_BIAS * LO_SCALE), lo);
+                        const float2 in = __ffma2_rn(lo,
                                                      make_float2(lo_unscale, lo_unscale),
                                                      make_float2(hh[u].x * unscale[u], hh[u].y * unscale[u]));
                         Step::step(s2[u], p2[u], in, n0, n1, K, o);
@@ -393,19 +432,20 @@ cudaError_t launch_ks(const IntegrateArgs &a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Compiled K extents; a run takes the least that holds its nodes.
-template <class M>
+// Compiled K extents; a run takes the least that holds its nodes.  X is the model above 80
+// nodes, Z above 128.
+template <class M, class X, class Z>
 cudaError_t launch_model(const IntegrateArgs &a, cudaStream_t st) {
     const int mt = (a.nodes + 15) / 16;
     if (mt <= 2) return launch_ks<M, 2>(a, st);
     if (mt <= 4) return launch_ks<M, 4>(a, st);
     if (mt <= 5) return launch_ks<M, 5>(a, st);
-    if (mt <= 6) return launch_ks<M, 6>(a, st);
-    if (mt <= 7) return launch_ks<M, 7>(a, st);
-    if (mt <= 8) return launch_ks<M, 8>(a, st);
-    if (mt <= 10) return launch_ks<M, 10>(a, st);
-    if (mt <= 13) return launch_ks<M, 13>(a, st);
-    if (mt <= 14) return launch_ks<M, 14>(a, st);
+    if (mt <= 6) return launch_ks<X, 6>(a, st);
+    if (mt <= 7) return launch_ks<X, 7>(a, st);
+    if (mt <= 8) return launch_ks<X, 8>(a, st);
+    if (mt <= 10) return launch_ks<Z, 10>(a, st);
+    if (mt <= 13) return launch_ks<Z, 13>(a, st);
+    if (mt <= 14) return launch_ks<Z, 14>(a, st);
     return cudaErrorInvalidValue;
 }
 
@@ -432,12 +472,19 @@ void fill_k32(int model, const ModelK &K, float *k32) {
     }
 }
 
+// The rates by rate2_acc where FP32 sums or better ones were there before, so that no run is
+// farther from FP64 than it was: BOLD, relative, geometric mean of 4-6 batches of 40 at
+// densities 0.25 / 0.8, per-simulation kernel (FP32 sums, expm1), fast rates, as here: rWW
+// 200 nodes 2.46e-8 / 2.30e-8, 3.03e-8 / 2.88e-8, 2.41e-8 / 2.28e-8; rWWEx 200 nodes 1.34e-7 /
+// 1.87e-7, 1.61e-7 / 2.05e-7, 1.18e-7 / 1.48e-7; WC 200 nodes 3.15e-8 / 3.12e-8, as here 2.02e-8 /
+// 2.03e-8; rWWEx 128 nodes 2.87e-7 / 1.69e-7 (tcgen05, BF16 halves), 1.70e-7 / 2.10e-7 with the
+// fast rate.  They cost 10-17 % (rWW 200 nodes 18.4 -> 20.0 ms per simulated second).
 cudaError_t launch_integrate_mma(int model, const IntegrateArgs &a, cudaStream_t st) {
     switch (model) {
-        case MODEL_RWW: return launch_model<RWW32>(a, st);
-        case MODEL_WC: return launch_model<WC32>(a, st);
-        case MODEL_JR: return launch_model<JR32>(a, st);
-        case MODEL_RWWEX: return launch_model<RWWEx32>(a, st);
+        case MODEL_RWW: return launch_model<RWW32, RWW32, RWW32T<true>>(a, st);
+        case MODEL_WC: return launch_model<WC32, WC32, WC32>(a, st);
+        case MODEL_JR: return launch_model<JR32, JR32, JR32>(a, st);
+        case MODEL_RWWEX: return launch_model<RWWEx32, RWWExs32, RWWExs32>(a, st);
         default: break;
     }
     return cudaErrorNotSupported;

@@ -172,7 +172,33 @@ __device__ __forceinline__ float2 rate2(float2 x, float d, float id, float ml2d)
     return make_float2(fabsf(y.x) < 1e-3f ? small.x : big.x, fabsf(y.y) < 1e-3f ? small.y : big.y);
 }
 
-struct RWW32 {  // rww.cpp:194-232 in FP32
+// The same to about an ulp: the Taylor series of y / (1 - e^-y) (Bernoulli numbers) to y^10
+// for |y| < 1.25 (first omitted term below 8e-9), beyond it with the exponent's rounding
+// error carried into the exponential.  y is capped where the rate is below 1e-33 of x, so
+// that the divisor stays finite.
+__device__ __forceinline__ float2 rate2_acc(float2 x, float d, float id) {
+    const float2 y = __fmul2_rn(x, f2(d)), w = __fmul2_rn(y, y);
+    float2 s = __ffma2_rn(w, f2(1.0f / 47900160.0f), f2(-1.0f / 1209600.0f));
+    s = __ffma2_rn(s, w, f2(1.0f / 30240.0f));
+    s = __ffma2_rn(s, w, f2(-1.0f / 720.0f));
+    s = __ffma2_rn(s, w, f2(1.0f / 12.0f));
+    s = __ffma2_rn(s, w, __ffma2_rn(y, f2(0.5f), f2(1.0f)));
+    const float2 small = __fmul2_rn(s, f2(id));
+    const float2 c = make_float2(fmaxf(y.x, -80.0f), fmaxf(y.y, -80.0f));
+    const float2 t = __fmul2_rn(c, f2(-1.44269502f));                       // log2(e) = 1.44269502 + 1.9259630e-8
+    float2 tl = __ffma2_rn(c, f2(-1.44269502f), make_float2(-t.x, -t.y));
+    tl = __ffma2_rn(c, f2(-1.9259630e-8f), tl);
+    const float2 e0 = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+    const float2 e = __ffma2_rn(__fmul2_rn(e0, tl), f2(0.693147181f), e0);
+    const float2 den = __ffma2_rn(e, f2(-1.0f), f2(1.0f));
+    const float2 big = __fmul2_rn(x, make_float2(rcp_approx(den.x), rcp_approx(den.y)));
+    return make_float2(fabsf(y.x) < 1.25f ? small.x : big.x, fabsf(y.y) < 1.25f ? small.y : big.y);
+}
+
+// ACC: the rates by rate2_acc.
+template <bool ACC_>
+struct RWW32T {  // rww.cpp:194-232 in FP32
+    static constexpr bool ACC = ACC_;
     static constexpr int NP = 5, NS = 2, NN = 2, NOUT = 6, CV = 0, BV = 0;
     struct K { float wEI0, wII0, aE, bE, dE, idE, aI, bI, dI, idI, wII, dgE, ditE, dgI, ditI, sqdt, ml2dE, ml2dI; };
     __host__ __device__ static K make(const ModelK &m) {
@@ -207,8 +233,9 @@ struct RWW32 {  // rww.cpp:194-232 in FP32
         IE = __ffma2_rn(p[3], sI, IE);
         float2 II = __ffma2_rn(p[2], sE, f2(k.wII0));
         II = __ffma2_rn(f2(-k.wII), sI, II);
-        const float2 rE = rate2(__ffma2_rn(f2(k.aE), IE, f2(-k.bE)), k.dE, k.idE, k.ml2dE);
-        const float2 rI = rate2(__ffma2_rn(f2(k.aI), II, f2(-k.bI)), k.dI, k.idI, k.ml2dI);
+        const float2 xE = __ffma2_rn(f2(k.aE), IE, f2(-k.bE)), xI = __ffma2_rn(f2(k.aI), II, f2(-k.bI));
+        const float2 rE = ACC ? rate2_acc(xE, k.dE, k.idE) : rate2(xE, k.dE, k.idE, k.ml2dE);
+        const float2 rI = ACC ? rate2_acc(xI, k.dI, k.idI) : rate2(xI, k.dI, k.idI, k.ml2dI);
         float2 dE = __fmul2_rn(f2(n0), p[4]);
         dE = __ffma2_rn(f2(k.dgE), __fmul2_rn(__ffma2_rn(sE, f2(-1.0f), f2(1.0f)), rE), dE);
         dE = __ffma2_rn(f2(-k.ditE), sE, dE);
@@ -220,6 +247,7 @@ struct RWW32 {  // rww.cpp:194-232 in FP32
         o[0] = IE; o[1] = II; o[2] = rE; o[3] = rI; o[4] = s[0]; o[5] = s[1];
     }
 };
+using RWW32 = RWW32T<false>;
 
 // Pair form for models without a packed step: two scalar steps.
 template <class M, bool = M::PAIR>
@@ -250,7 +278,7 @@ struct PairStep<M, true> {
 };
 
 struct WC32 {  // wc.cpp:51-80 in FP32
-    static constexpr bool PAIR = false;
+    static constexpr bool PAIR = false, ACC = false;
     static constexpr int NP = 9, NS = 2, NN = 2, NOUT = 2, CV = 0, BV = 0;
     struct K { float dt, sqdt, itE, itI, aE, aI, muE, muI; };
     __host__ __device__ static K make(const ModelK &m) {
@@ -276,7 +304,7 @@ struct WC32 {  // wc.cpp:51-80 in FP32
 };
 
 struct RWWEx32 {  // rwwex.cpp:48-73 in FP32
-    static constexpr bool PAIR = false;
+    static constexpr bool PAIR = false, ACC = false;
     static constexpr int NP = 4, NS = 1, NN = 1, NOUT = 3, CV = 0, BV = 0;
     struct K { float JN, a, b, d, id, dit, dg, sqdt; };
     __host__ __device__ static K make(const ModelK &m) {
@@ -297,7 +325,7 @@ struct RWWEx32 {  // rwwex.cpp:48-73 in FP32
 };
 
 struct JR32 {  // jr.cpp:80-133 in FP32
-    static constexpr bool PAIR = false;
+    static constexpr bool PAIR = false, ACC = false;
     static constexpr int NP = 7, NS = 8, NN = 1, NOUT = 8, CV = 7, BV = 6;
     struct K { float dt, sqdt, A, B, a, b, v0, numax2, r, mu, cmin, cmax, mid, asq, bsq; };
     __host__ __device__ static K make(const ModelK &m) {
