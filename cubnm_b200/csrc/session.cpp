@@ -840,6 +840,19 @@ static int tuned_variant(const cbnm_run_args *a, const Cfg &c, const std::string
     return best_v;
 }
 
+// Most nonzeros in a column of any SC (the sources of one target).
+static int longest_column(const double *sc, int n_scs, int n) {
+    int most = 0;
+    std::vector<int> cnt(n);
+    for (int s = 0; s < n_scs; ++s) {
+        std::fill(cnt.begin(), cnt.end(), 0);
+        for (int k = 0; k < n; ++k)
+            for (int j = 0; j < n; ++j) cnt[j] += sc[((size_t)s * n + k) * n + j] != 0.0;
+        most = std::max(most, *std::max_element(cnt.begin(), cnt.end()));
+    }
+    return most;
+}
+
 // tan_bold (device, [N][bold_len][nodes]) non-null: also integrate the tangent along
 // G and write dBOLD/dG there (lane kernel, FP32 precision, rWW or WC).
 static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool device_io, double *tan_bold) {
@@ -1007,9 +1020,53 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         if (!ok) throw Err(CBNM_ERR_UNSUPPORTED, std::string("integrator variant ") + kVariantName[variant] +
                                                      " does not apply to this run");
     }
+    // host copies of the SCs and of the simulations' SC indices, fetched on first use
+    std::vector<double> sc_copy;
+    auto host_sc = [&]() -> const double * {
+        if (!device_io) return a->sc;
+        if (sc_copy.empty()) {
+            sc_copy.resize(nn * a->n_scs);
+            CK(cudaMemcpy(sc_copy.data(), a->sc, sizeof(double) * sc_copy.size(), cudaMemcpyDeviceToHost));
+        }
+        return sc_copy.data();
+    };
+    auto host_sc_idx = [&]() -> const int * {
+        if (!device_io) return a->sc_indices;
+        if (h_sc_idx.size() != (size_t)N) {
+            h_sc_idx.resize(N);
+            CK(cudaMemcpy(h_sc_idx.data(), a->sc_indices, sizeof(int) * N, cudaMemcpyDeviceToHost));
+        }
+        return h_sc_idx.data();
+    };
     // (CBNM_FP32_KERNEL=lanes leaves networks the 32-wide tiles hold, <= 128 nodes, on the tiles)
-    const bool use_tc = variant == V_DEFAULT ? (!tan_bold && !force_simt && tc_ok && !(force_lanes && n > 128))
+    bool use_tc = variant == V_DEFAULT ? (!tan_bold && !force_simt && tc_ok && !(force_lanes && n > 128))
                                              : (variant == V_PP || variant == V_PPWS || variant == V_V5);
+    // Above 128 nodes tiles with few simulations each (an SC for every one or two of them)
+    // can take longer than the per-simulation kernel.  ms per simulated second: a wave of
+    // tiles 0.095 n (rWW 136 nodes 12.9, 200 nodes 20.0, 224 nodes 21.1); 148 simulations one
+    // by one (0.02 + 0.17 k / n) n with sparse coupling of at most k sources (200 nodes,
+    // density 0.1 9.8, 0.3 17.5, where a table stays in the L1), 0.115 n dense (24); packing the
+    // sparse tables 7 ns an SC entry on the host.  512 simulations of 200 nodes with an SC
+    // each: tiles 80, one by one 34 at density 0.1, 60 at 0.3, 84 at 0.8.
+    if (use_tc && variant == V_DEFAULT && n > 128 && !num_fic) {
+        std::vector<int> count(a->n_scs, 0);
+        const int *of = host_sc_idx();
+        for (int s = 0; s < N; ++s) {
+            if (of[s] < 0 || of[s] >= a->n_scs) throw Err(CBNM_ERR_ARG, "SC index out of range");
+            ++count[of[s]];
+        }
+        long long tiles = 0;
+        for (int k : count) tiles += (k + FP32_TILE - 1) / FP32_TILE;
+        if (4 * tiles > N && !std::getenv("CBNM_COUPLING")) {
+            const int k = longest_column(host_sc(), a->n_scs, n), sms = sm_count();
+            const bool sparse = 2 * k <= n;
+            const double secs = c.bw_it * (double)c.inner_it * 1e-4;   // in steps of 0.1 ms
+            const double one = !sparse ? 0.115 : (size_t)k * n * 8 <= 150 * 1024 ? 0.02 + 0.17 * k / n : 0.18;
+            const double tiles_ms = secs * 0.095 * n * (double)((tiles + sms - 1) / sms);
+            const double sims_ms = secs * one * n * std::max(1.3, (double)N / sms) + (sparse ? 7e-6 * a->n_scs * nn : 0.0);
+            if (sims_ms < tiles_ms) use_tc = false;
+        }
+    }
     bool use_lanes = variant == V_DEFAULT ? (lanes_ok && (tan_bold || (force_lanes && !use_tc)))
                                           : (variant == V_LANES || variant == V_LANES512);
     const int lanes_threads = variant == V_LANES512 ? 512 : 1024;
@@ -1023,19 +1080,9 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     // delays are below a block, and FP64 networks whose rows do not fit shared memory.
     DelayPlan plan;
     bool delay_blocks = has_delay && !md.osc && !use_lanes && !force_simt && !std::getenv("CBNM_COUPLING");
-    const double *sc_host = h_sc;
-    std::vector<double> sc_copy;
-    if (has_delay && device_io) {
-        sc_copy.resize(nn * a->n_scs);
-        CK(cudaMemcpy(sc_copy.data(), a->sc, sizeof(double) * sc_copy.size(), cudaMemcpyDeviceToHost));
-        sc_host = sc_copy.data();
-        if (h_sc_idx.size() != (size_t)N) {
-            h_sc_idx.resize(N);
-            CK(cudaMemcpy(h_sc_idx.data(), a->sc_indices, sizeof(int) * N, cudaMemcpyDeviceToHost));
-        }
-    }
     if (delay_blocks) {
-        const int *sc_of = device_io ? h_sc_idx.data() : a->sc_indices;
+        const int *sc_of = host_sc_idx();
+        const double *sc_host = host_sc();
         const int dmax = *std::max_element(h_max_delay.begin(), h_max_delay.end());
         const size_t most = (size_t)1 << 30;
         delay_blocks = c.fp32 ? build_delay_plan<float>(plan, n, N, md.n_noise, sm_count(), sc_host, sc_of, h_delay,
@@ -1173,20 +1220,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         // nonzeros summed in ascending source order, so FP64 sums are unchanged.
         // The packed ring-buffer offsets are 32-bit: every simulation's buffer must
         // hold fewer than 2^30 values, else the dense loop runs.
-        std::vector<double> sc_host;
-        const double *src = h_sc;
-        if (device_io) {
-            sc_host.resize(nn * a->n_scs);
-            CK(cudaMemcpy(sc_host.data(), a->sc, sizeof(double) * sc_host.size(), cudaMemcpyDeviceToHost));
-            src = sc_host.data();
-        }
-        int kmax = 0;
-        for (int sc = 0; sc < a->n_scs; ++sc)
-            for (int j = 0; j < n; ++j) {
-                int cnt = 0;
-                for (int k = 0; k < n; ++k) cnt += src[(size_t)sc * nn + (size_t)k * n + j] != 0.0;
-                kmax = std::max(kmax, cnt);
-            }
+        const double *src = host_sc();
+        const int kmax = longest_column(src, a->n_scs, n);
         const char *cpl = std::getenv("CBNM_COUPLING");
         const std::string mode = cpl ? cpl : "";
         const long long max_hist = has_delay ? (long long)*std::max_element(h_max_delay.begin(), h_max_delay.end()) * n : 0;
@@ -1252,16 +1287,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     const bool pp_ws = use_pp && (variant == V_DEFAULT ? (tc_kind && std::string(tc_kind) == "ws") : variant == V_PPWS);
     // tiles of TN simulations that share one SC: [n][1 + TN] = SC index, simulation ids (-1 = empty)
     auto make_tiles = [&](int TN) {
-        std::vector<int> sc_of(N);
-        if (device_io) {
-            if (h_sc_idx.size() != (size_t)N) {
-                h_sc_idx.resize(N);
-                CK(cudaMemcpy(h_sc_idx.data(), a->sc_indices, sizeof(int) * N, cudaMemcpyDeviceToHost));
-            }
-            sc_of.assign(h_sc_idx.begin(), h_sc_idx.end());
-        } else {
-            sc_of.assign(a->sc_indices, a->sc_indices + N);
-        }
+        const int *sc_of = host_sc_idx();
         std::vector<int> order(N);
         std::iota(order.begin(), order.end(), 0);
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return sc_of[x] < sc_of[y]; });
@@ -1306,16 +1332,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     } else if (use_lanes) {
         // groups of 16 simulations sharing SC and delay table (bnm.cu runs one
         // CTA per simulation; here one CTA integrates a group)
-        std::vector<int> sc_of(N);
-        if (device_io) {
-            if (h_sc_idx.size() != (size_t)N) {
-                h_sc_idx.resize(N);
-                CK(cudaMemcpy(h_sc_idx.data(), a->sc_indices, sizeof(int) * N, cudaMemcpyDeviceToHost));
-            }
-            sc_of.assign(h_sc_idx.begin(), h_sc_idx.end());
-        } else {
-            sc_of.assign(a->sc_indices, a->sc_indices + N);
-        }
+        const int *sc_of = host_sc_idx();
         std::vector<int> order(N);
         std::iota(order.begin(), order.end(), 0);
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) {

@@ -8,11 +8,11 @@ from cubnm_b200 import core
 pytestmark = pytest.mark.gpu
 
 
-def _run(model, nodes, N, precision, velocity=0.0, density=0.3, scs=1, **config):
+def _run(model, nodes, N, precision, velocity=0.0, density=0.3, scs=1, ms=100, **config):
     a = list(cases.synthetic_args(model, N=N, nodes=nodes, duration_s=1, seed=nodes, density=density,
                                   G=np.linspace(0.2, 1.2, N), bold_remove_s=0, do_fcd=False, precision=precision))
     a[7] = dict(a[7], do_fc="0", noise_time_steps="100", **config)
-    a[16], a[17], a[18] = 100, 100, 100
+    a[16], a[17], a[18] = ms, 100, 100
     if scs > 1:
         a[1] = np.stack([cases.synthetic_sc(nodes, density, s).reshape(-1) for s in range(scs)])
         a[2] = (np.arange(N) % scs).astype(np.intc)
@@ -48,6 +48,15 @@ def test_fp64_form_by_waves(nodes, N, scs, kernel):
     ("rWW", 900, "fp64", 0.1, "k_integrate_sim"), ("Kuramoto", 60, "fp64", 0.2, "k_integrate_sim")])
 def test_with_delays(model, nodes, precision, density, kernel):
     assert _run(model, nodes, 3, precision, velocity=6.0, density=density) == kernel
+
+
+@pytest.mark.parametrize("nodes,N,scs,density,kernel", [
+    (200, 300, 1, 0.1, "k_integrate_mma"), (200, 300, 300, 0.1, "k_integrate_sim"),
+    (200, 148, 148, 0.8, "k_integrate_mma"), (128, 300, 300, 0.1, "k_integrate_mma")])
+def test_fp32_tiles_by_their_filling(nodes, N, scs, density, kernel):
+    """Above 128 nodes a sparse SC for every simulation leaves the tiles in a run that is long enough for
+    packing the sparse tables on the host not to count."""
+    assert _run("rWW", nodes, N, "fp32", scs=scs, density=density, ms=3000) == kernel
 
 
 def test_forced_kernels(monkeypatch):
