@@ -36,20 +36,25 @@ inline std::vector<std::pair<int, int>> delay_pairs(DelayPlan &p, int n_sims, co
     return pairs;
 }
 
-// A tile's entry lists (per pass over the targets), 16-byte aligned: this header, unsigned end[targets] (low half: pairs of
-// far entries up to and with the target's, high half: near entries), then at the byte
-// offsets given: far offsets into the tile's windows of x(t0 - d) (16 bits each, a
-// target's padded to a pair by repeating one with weight 0), their weights, near codes
-// (offset * 32 + delay) and their weights.
-struct TileHead { int off_at, w_at, near_at, near_w_at; };
+// Words between the windows of two sources in shared memory: a window of p.window steps
+// before the block, then DELAY_BLOCK zeros, where the lanes b >= d of a pair with
+// d < DELAY_BLOCK read (their values are not there yet; the step loop adds them).
+inline int delay_stride(int window) { return window + DELAY_BLOCK; }
 
-// Lists of all pairs for tiles of p.tile_src sources; R = float or double.  False
-// where a list exceeds its index width or all lists max_bytes.
+// A tile's entry lists (per pass over the targets), 16-byte aligned: this header, unsigned
+// end[targets] (pairs of entries up to and with the target's), then at the byte offsets
+// given the offsets of x(t0 - d) in the tile's windows (16 bits each, a target's padded to a
+// pair by repeating one with weight 0) and the weights.  A target's sources are in ascending
+// order, so that its sum over all tiles is one chain in that order whatever the tiles are.
+struct TileHead { int off_at, w_at, unused[2]; };
+
+// Lists of all pairs for tiles of p.tile_src sources; R = float or double.  False where all
+// lists exceed max_bytes.
 template <class R>
 inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector<int> &delay,
                         const std::vector<std::pair<int, int>> &pairs, size_t max_bytes) {
     const size_t nn = (size_t)n * n;
-    const int W = p.window;
+    const int W = p.window, WS = delay_stride(W);
     p.tiles = (n + p.tile_src - 1) / p.tile_src;
     p.blob.clear();
     p.blob_at.clear();
@@ -57,8 +62,7 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
     const int nh = (n + p.passes - 1) / p.passes;
     std::vector<unsigned> end(nh);
     std::vector<uint16_t> off;
-    std::vector<int> noff;
-    std::vector<R> w, nw;
+    std::vector<R> w;
     auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
     for (const auto &pr : pairs) {
         const double *S = sc + (size_t)pr.first * nn;
@@ -66,33 +70,25 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
         for (int pt = 0; pt < p.passes * p.tiles; ++pt) {
             const int pass = pt / p.tiles, t = pt % p.tiles;
             const int s0 = t * p.tile_src, s1 = std::min(n, s0 + p.tile_src), h0 = pass * nh, h1 = std::min(n, h0 + nh);
-            off.clear(); w.clear(); noff.clear(); nw.clear();
+            off.clear();
+            w.clear();
             for (int j = h0; j < h1; ++j) {
                 for (int k = s0; k < s1; ++k) {
                     const double v = S[(size_t)k * n + j];
                     if (v == 0.0) continue;
-                    const int dk = d[(size_t)k * n + j], o = (k - s0) * W + (W - dk);
-                    if (dk >= DELAY_BLOCK) {
-                        off.push_back((uint16_t)o);
-                        w.push_back((R)v);
-                    } else {
-                        noff.push_back(o * 32 + dk);
-                        nw.push_back((R)v);
-                    }
+                    off.push_back((uint16_t)((k - s0) * WS + (W - d[(size_t)k * n + j])));
+                    w.push_back((R)v);
                 }
                 if (off.size() % 2) {
                     off.push_back(off.back());
                     w.push_back(R(0));
                 }
-                if (off.size() / 2 > 0xffff || noff.size() > 0xffff) return false;
-                end[j - h0] = (unsigned)(off.size() / 2) | ((unsigned)noff.size() << 16);
+                end[j - h0] = (unsigned)(off.size() / 2);
             }
-            TileHead h;
+            TileHead h{};
             h.off_at = (int)up16(sizeof(h) + sizeof(unsigned) * nh);
             h.w_at = (int)up16(h.off_at + sizeof(uint16_t) * off.size());
-            h.near_at = (int)up16(h.w_at + sizeof(R) * w.size());
-            h.near_w_at = (int)up16(h.near_at + sizeof(int) * noff.size());
-            const size_t bytes = up16(h.near_w_at + sizeof(R) * nw.size()), at = p.blob.size();
+            const size_t bytes = up16(h.w_at + sizeof(R) * w.size()), at = p.blob.size();
             p.blob_at.push_back((int)(at / 16));
             p.blob.resize(at + bytes);
             unsigned char *b = p.blob.data() + at;
@@ -101,10 +97,6 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
             if (!off.empty()) {
                 std::memcpy(b + h.off_at, off.data(), sizeof(uint16_t) * off.size());
                 std::memcpy(b + h.w_at, w.data(), sizeof(R) * w.size());
-            }
-            if (!noff.empty()) {
-                std::memcpy(b + h.near_at, noff.data(), sizeof(int) * noff.size());
-                std::memcpy(b + h.near_w_at, nw.data(), sizeof(R) * nw.size());
             }
             p.blob_max = std::max(p.blob_max, (int)bytes);
             if (p.blob.size() > max_bytes) return false;
@@ -127,44 +119,53 @@ inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int s
     p.window = (std::max(max_delay, DELAY_BLOCK) + DELAY_BLOCK - 1) / DELAY_BLOCK * DELAY_BLOCK;
     const auto pairs = delay_pairs(p, n_sims, sc_of, table_of);
     const size_t nn = (size_t)n * n;
-    // near lists for the steps within a block, by rank q
+    // near lists (d < DELAY_BLOCK) for the steps within a block, by rank q: counted first
     p.near_cnt.assign(p.n_pairs, 0);
     p.near_min.assign(p.n_pairs, DELAY_BLOCK);
-    struct Near { int pair, node, rank, off; double w; };
-    std::vector<Near> near;
     size_t nnz = 0;   // of the fullest pair
     if ((size_t)p.n_pairs * nn > max_bytes) return false;
+    std::vector<int> near(n), all(n);
     for (int q = 0; q < p.n_pairs; ++q) {
         const double *S = sc + (size_t)pairs[q].first * nn;
         const int *d = delay.data() + (size_t)pairs[q].second * nn;
-        size_t all = 0;
-        for (int j = 0; j < n; ++j) {
-            int rank = 0, far = 0;
-            for (int k = 0; k < n; ++k) {
-                const double v = S[(size_t)k * n + j];
-                if (v == 0.0) continue;
+        std::fill(near.begin(), near.end(), 0);
+        std::fill(all.begin(), all.end(), 0);
+        for (int k = 0; k < n; ++k)
+            for (int j = 0; j < n; ++j) {
+                if (S[(size_t)k * n + j] == 0.0) continue;
                 const int dk = d[(size_t)k * n + j];
-                if (dk >= DELAY_BLOCK) { ++far; continue; }
-                near.push_back({q, j, rank++, k * DELAY_BLOCK + dk, v});
+                ++all[j];
+                if (dk >= DELAY_BLOCK) continue;
+                ++near[j];
                 p.near_min[q] = std::min(p.near_min[q], dk);
             }
-            p.near_cnt[q] = std::max(p.near_cnt[q], rank);
-            p.far_max = std::max(p.far_max, far);
-            all += far + rank;
-        }
-        nnz = std::max(nnz, all);
+        p.near_cnt[q] = *std::max_element(near.begin(), near.end());
+        p.far_max = std::max(p.far_max, *std::max_element(all.begin(), all.end()) - p.near_cnt[q]);
+        size_t sum = 0;
+        for (int c : all) sum += c;
+        nnz = std::max(nnz, sum);
     }
     for (int c : p.near_cnt) p.near_k = std::max(p.near_k, c);
     if (p.near_k > std::max(8, p.far_max / 4) || (size_t)p.n_pairs * p.near_k * n * 16 > max_bytes) return false;
     p.near.assign((size_t)p.n_pairs * p.near_k * n, 0);
     p.near_w.assign(p.near.size(), 0.0);
-    for (const Near &e : near) {
-        const size_t at = ((size_t)e.pair * p.near_k + e.rank) * n + e.node;
-        p.near[at] = e.off;
-        p.near_w[at] = e.w;
+    for (int q = 0; q < p.n_pairs; ++q) {
+        const double *S = sc + (size_t)pairs[q].first * nn;
+        const int *d = delay.data() + (size_t)pairs[q].second * nn;
+        if (p.near_cnt[q] == 0) continue;
+        std::fill(near.begin(), near.end(), 0);
+        for (int k = 0; k < n; ++k)
+            for (int j = 0; j < n; ++j) {
+                const double v = S[(size_t)k * n + j];
+                const int dk = d[(size_t)k * n + j];
+                if (v == 0.0 || dk >= DELAY_BLOCK) continue;
+                const size_t at = ((size_t)q * p.near_k + near[j]++) * n + j;
+                p.near[at] = k * DELAY_BLOCK + dk;
+                p.near_w[at] = v;
+            }
     }
     // tile and launch shape
-    const int least = (n + 31) / 32 * 32;
+    const int least = (n + 31) / 32 * 32, stride = delay_stride(p.window);
     const bool f64 = sizeof(R) == 8;
     const int rows = (int)(sizeof(R) * n * (DELAY_BLOCK + 1) + 15) & ~15;
     const double nnz_node = (double)nnz / n;
@@ -174,8 +175,8 @@ inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int s
         const int most_smem = DELAY_SMEM_SM / c - 1024;
         auto fit = [&](int bufs) {   // sources whose windows and entries, with row ends and padding, fill a buffer
             const double fixed = (double)n / p.passes * (4 + 0.6 * (2 + sizeof(R))) + 512;
-            const double src = (double)p.window * sizeof(R) + nnz_node / p.passes * 1.1 * (2 + sizeof(R));
-            return std::min<int>({n, 65535 / p.window, (int)(((most_smem - p.buf_at) / bufs - fixed) / src)});
+            const double src = (double)stride * sizeof(R) + nnz_node / p.passes * 1.1 * (2 + sizeof(R));
+            return std::min<int>({n, 65535 / stride, (int)(((most_smem - p.buf_at) / bufs - fixed) / src)});
         };
         p.bufs = p.passes = 1;
         p.buf_at = p.noise_at = rows;
@@ -196,7 +197,7 @@ inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int s
         p.threads = std::max(least, most);
         for (int shrink = 0; shrink < 8 && p.tile_src >= 1; ++shrink) {
             if (!delay_blobs<R>(p, n, sc, delay, pairs, max_bytes)) return false;
-            p.buf_bytes = ((p.blob_max + p.tile_src * p.window * (int)sizeof(R)) + 15) & ~15;
+            p.buf_bytes = ((p.blob_max + p.tile_src * stride * (int)sizeof(R)) + 15) & ~15;
             p.smem = p.buf_at + p.bufs * p.buf_bytes;
             if (p.smem <= most_smem) {
                 if (p.passes == 2) p.smem = most_smem & ~15;

@@ -149,7 +149,7 @@ struct IntegrateArgs {
     const int4 *ell_pk64;        // [n_scs][ell_tables][ell_k][nodes] {weight lo, weight hi, offset, 0} (FP64 kernel)
     // Delay kernel (integrate_delay.cuh; lists from delay_plan.h), per used (SC, delay
     // table) pair.  Ring buffers [CTA][node][db_window] in hist / hist_f32.
-    int db_window;               // slots per node: the largest delay rounded up to 32
+    int db_window;               // slots per node: the largest delay rounded up to 32 (32 zeros follow them in a buffer)
     int db_tiles, db_tile_src;   // source tiles, and sources per tile
     int db_bufs;                 // tile buffers in shared memory (2: the next tile loads during this one)
     int db_blob_max;             // bytes reserved for a tile's entry lists in a buffer

@@ -12,7 +12,7 @@
 //     lists; a warp takes target node j and runs over the nonzeros of its SC column
 //     within the tile; its 32 lanes read x_k(t0 + b - d), b = 0..31, 32 consecutive
 //     words, and accumulate w x.  Pairs with d >= 32 ("far") need only values from
-//     before t0; of the others ("near") the lanes b < d take part.
+//     before t0; of the others ("near") the lanes b >= d read zeros behind the window.
 //  2. steps: thread j integrates node j through the 32 steps with the sums of 1
 //     in shared memory, adding the near pairs' terms with b >= d from the values
 //     this block has already produced.  Those are read by other threads, so a
@@ -28,8 +28,9 @@
 // steps, half a wavefront for the entry itself), step 2 the latency of the update's
 // dependency chain.  Gathering straight from global memory through L1 took 5.3 cycles
 // an entry (the 128-byte window is unaligned: two lines, five sectors) against about
-// 1.5 from shared memory.  The sums run over the source tiles, in each the far pairs,
-// then the near pairs, each in ascending source order (before: one ascending order).
+// 1.5 from shared memory.  A target's sum runs over its sources in ascending order, then
+// over the near pairs whose value the block has produced, so that it depends neither on the
+// tiles nor on what else is in the batch.
 #pragma once
 #include <algorithm>
 #include "delay_plan.h"
@@ -94,14 +95,15 @@ __device__ __forceinline__ void stage_tile(const IntegrateArgs &a, int pair, int
     const int4 *src = reinterpret_cast<const int4 *>(a.db_blob) + b0;
     for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) cp16(buf + 16 * (size_t)i, src + i);
     R *win = reinterpret_cast<R *>(buf + a.db_blob_max);
-    const int W = a.db_window, s0 = t * a.db_tile_src, cnt = min(a.db_tile_src, a.nodes - s0);
+    const int W = a.db_window, WS = W + DB, s0 = t * a.db_tile_src, cnt = min(a.db_tile_src, a.nodes - s0);
     constexpr int V = 16 / sizeof(R);
     for (int k = warp; k < cnt; k += nwarps) {
         const R *h = hist + (size_t)(s0 + k) * W;
+        win[(size_t)k * WS + W + lane] = R(0);   // where the steps of a near pair read that the block has not done
         for (int c = lane * V; c < W; c += 32 * V) {
             int p = t0m + c;
             if (p >= W) p -= W;
-            cp16(win + (size_t)k * W + c, h + p);
+            cp16(win + (size_t)k * WS + c, h + p);
         }
     }
 }
@@ -157,11 +159,10 @@ __device__ __noinline__ void gather_block(const IntegrateArgs &a, int pair, int 
         const unsigned *off = reinterpret_cast<const unsigned *>(buf + head->off_at);   // two 16-bit offsets a word
         const R *wgt = reinterpret_cast<const R *>(buf + head->w_at);
         const R *win = reinterpret_cast<const R *>(buf + a.db_blob_max) + lane;
-        const unsigned before = k0 > 0 ? rend[k0 - 1] : 0;
-        unsigned p = before & 0xffff, pn = before >> 16;   // in pairs of far entries, in near entries
+        unsigned p = k0 > 0 ? rend[k0 - 1] : 0;   // in pairs of entries
         for (int k = k0; k < k1; ++k) {
-            const unsigned e = rend[k], pe = e & 0xffff, ne = e >> 16;
-            if (t > 0 && p == pe && pn == ne) continue;
+            const unsigned pe = rend[k];
+            if (t > 0 && p == pe) continue;
             R acc = t == 0 ? R(0) : row[k * DROW + lane];
 #pragma unroll 4
             for (; p < pe; ++p) {
@@ -170,11 +171,6 @@ __device__ __noinline__ void gather_block(const IntegrateArgs &a, int pair, int 
                 A::pair(wgt, p, w0, w1);
                 acc = A::mad(w0, win[o & 0xffff], acc);
                 acc = A::mad(w1, win[o >> 16], acc);
-            }
-            for (; pn < ne; ++pn) {   // near pairs: the steps before their values are in the block
-                const int o = reinterpret_cast<const int *>(buf + head->near_at)[pn];
-                if (lane < (o & (DB - 1)))
-                    acc = A::mad(reinterpret_cast<const R *>(buf + head->near_w_at)[pn], win[o >> 5], acc);
             }
             row[k * DROW + lane] = acc;
         }
