@@ -1038,6 +1038,9 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         }
         return h_sc_idx.data();
     };
+    // "dense" or "sparse" asks for the per-step kernels with that coupling form
+    const char *coupling = std::getenv("CBNM_COUPLING");
+    const bool coupling_forced = coupling && (std::string(coupling) == "dense" || std::string(coupling) == "sparse");
     // (CBNM_FP32_KERNEL=lanes leaves networks the 32-wide tiles hold, <= 128 nodes, on the tiles)
     bool use_tc = variant == V_DEFAULT ? (!tan_bold && !force_simt && tc_ok && !(force_lanes && n > 128))
                                              : (variant == V_PP || variant == V_PPWS || variant == V_V5);
@@ -1057,7 +1060,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         }
         long long tiles = 0;
         for (int k : count) tiles += (k + FP32_TILE - 1) / FP32_TILE;
-        if (4 * tiles > N && !std::getenv("CBNM_COUPLING")) {
+        if (4 * tiles > N && !coupling_forced) {
             const int k = longest_column(host_sc(), a->n_scs, n), sms = sm_count();
             const bool sparse = 2 * k <= n;
             const double secs = c.bw_it * (double)c.inner_it * 1e-4;   // in steps of 0.1 ms
@@ -1079,7 +1082,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     // target's current phase, keeps the per-step loop, as do networks of which most
     // delays are below a block, and FP64 networks whose rows do not fit shared memory.
     DelayPlan plan;
-    bool delay_blocks = has_delay && !md.osc && !use_lanes && !force_simt && !std::getenv("CBNM_COUPLING");
+    bool delay_blocks = has_delay && !md.osc && !use_lanes && !force_simt && !coupling_forced;
     if (delay_blocks) {
         const int *sc_of = host_sc_idx();
         const double *sc_host = host_sc();
@@ -1211,7 +1214,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     }
     // FP64 without delays or numerical FIC, up to 128 nodes: the register-resident forms
     // (integrate_tile64.cu) unless a coupling form of the per-simulation kernel is forced.
-    const bool t64 = !c.fp32 && !has_delay && !num_fic && tile64_supported(md.id, n) && !std::getenv("CBNM_COUPLING");
+    const bool t64 = !c.fp32 && !has_delay && !num_fic && tile64_supported(md.id, n) && !coupling_forced;
     bool t64_tiles = false;
     if (!use_tc && !delay_blocks && !t64) {
         // Sparse coupling for the per-simulation kernels (ELLPACK by target node):
@@ -1222,8 +1225,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         // hold fewer than 2^30 values, else the dense loop runs.
         const double *src = host_sc();
         const int kmax = longest_column(src, a->n_scs, n);
-        const char *cpl = std::getenv("CBNM_COUPLING");
-        const std::string mode = cpl ? cpl : "";
+        const std::string mode = coupling ? coupling : "";
         const long long max_hist = has_delay ? (long long)*std::max_element(h_max_delay.begin(), h_max_delay.end()) * n : 0;
         const bool fits = max_hist < (1LL << 30);
         const bool sparse =

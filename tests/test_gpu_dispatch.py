@@ -67,3 +67,13 @@ def test_forced_kernels(monkeypatch):
     monkeypatch.delenv("CBNM_FP32_KERNEL")
     monkeypatch.setenv("CBNM_FP32_TC", "pp")
     assert _run("rWW", 100, 100, "fp32") == "k_integrate_pp"
+
+
+@pytest.mark.parametrize("value,fp64,delayed", [("auto", "k_one64", "k_integrate_delay"),
+                                                ("sparse", "k_integrate_sim", "k_integrate_sim"),
+                                                ("dense", "k_integrate_sim", "k_integrate_sim")])
+def test_coupling_form(value, fp64, delayed, monkeypatch):
+    """CBNM_COUPLING asks for the per-step kernels by naming a coupling form, not by being set."""
+    monkeypatch.setenv("CBNM_COUPLING", value)
+    assert _run("rWW", 60, 5, "fp64") == fp64
+    assert _run("rWW", 60, 5, "fp64", velocity=6.0) == delayed
