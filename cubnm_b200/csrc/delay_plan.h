@@ -14,8 +14,10 @@ constexpr int DELAY_SMEM_SM = 227 * 1024;   // shared memory of an SM that CTAs 
 
 struct DelayPlan {
     int window = 0, tiles = 0, tile_src = 0, bufs = 1, threads = 0, blob_max = 0, buf_bytes = 0, passes = 1, buf_at = 0, noise_at = 0, noise_steps = 0;
-    int smem = 0, n_pairs = 0, near_k = 1, far_max = 0;
-    std::vector<int> pair, blob_at, near, near_cnt, near_min;
+    int smem = 0, n_pairs = 0, near_k = 1;
+    std::vector<int> sims, pair;   // the simulations that run on the kernel, and each one's pair (as all of [n_sims])
+    std::vector<int> rest;         // the others: their pair is not for it
+    std::vector<int> blob_at, near, near_cnt, near_min;
     std::vector<unsigned char> blob;
     std::vector<double> near_w;
 };
@@ -48,11 +50,40 @@ inline int delay_stride(int window) { return window + DELAY_BLOCK; }
 // order, so that its sum over all tiles is one chain in that order whatever the tiles are.
 struct TileHead { int off_at, w_at, unused[2]; };
 
+// The nonzeros of one SC by target, sources ascending; loaded again only when the SC changes,
+// so that many delay tables of one SC are walked by their entries, not by all n x n.
+struct DelayColumns {
+    int loaded = -1;
+    int full = 0;               // most sources of a target
+    std::vector<int> at, src;   // target j: entries at[j] .. at[j + 1]
+    std::vector<double> w;
+    void load(const double *sc, int id, int n) {
+        if (id == loaded) return;
+        loaded = id;
+        const double *S = sc + (size_t)id * n * n;
+        at.assign(n + 1, 0);
+        for (int k = 0; k < n; ++k)
+            for (int j = 0; j < n; ++j) at[j + 1] += S[(size_t)k * n + j] != 0.0;
+        full = *std::max_element(at.begin(), at.end());
+        for (int j = 0; j < n; ++j) at[j + 1] += at[j];
+        src.resize(at[n]);
+        w.resize(at[n]);
+        std::vector<int> next(at.begin(), at.end() - 1);
+        for (int k = 0; k < n; ++k)
+            for (int j = 0; j < n; ++j) {
+                const double v = S[(size_t)k * n + j];
+                if (v == 0.0) continue;
+                src[next[j]] = k;
+                w[next[j]++] = v;
+            }
+    }
+};
+
 // Lists of all pairs for tiles of p.tile_src sources; R = float or double.  False where all
 // lists exceed max_bytes.
 template <class R>
 inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector<int> &delay,
-                        const std::vector<std::pair<int, int>> &pairs, size_t max_bytes) {
+                        const std::vector<std::pair<int, int>> &pairs, DelayColumns &cols, size_t max_bytes) {
     const size_t nn = (size_t)n * n;
     const int W = p.window, WS = delay_stride(W);
     p.tiles = (n + p.tile_src - 1) / p.tile_src;
@@ -61,23 +92,25 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
     p.blob_max = 0;
     const int nh = (n + p.passes - 1) / p.passes;
     std::vector<unsigned> end(nh);
+    std::vector<int> at(nh);   // a target's next entry: tiles take them in order
     std::vector<uint16_t> off;
     std::vector<R> w;
     auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
     for (const auto &pr : pairs) {
-        const double *S = sc + (size_t)pr.first * nn;
+        cols.load(sc, pr.first, n);
         const int *d = delay.data() + (size_t)pr.second * nn;
         for (int pt = 0; pt < p.passes * p.tiles; ++pt) {
             const int pass = pt / p.tiles, t = pt % p.tiles;
             const int s0 = t * p.tile_src, s1 = std::min(n, s0 + p.tile_src), h0 = pass * nh, h1 = std::min(n, h0 + nh);
+            if (t == 0) std::copy(cols.at.begin() + h0, cols.at.begin() + h1, at.begin());
             off.clear();
             w.clear();
             for (int j = h0; j < h1; ++j) {
-                for (int k = s0; k < s1; ++k) {
-                    const double v = S[(size_t)k * n + j];
-                    if (v == 0.0) continue;
+                int &e = at[j - h0];
+                for (; e < cols.at[j + 1] && cols.src[e] < s1; ++e) {
+                    const int k = cols.src[e];
                     off.push_back((uint16_t)((k - s0) * WS + (W - d[(size_t)k * n + j])));
-                    w.push_back((R)v);
+                    w.push_back((R)cols.w[e]);
                 }
                 if (off.size() % 2) {
                     off.push_back(off.back());
@@ -88,10 +121,10 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
             TileHead h{};
             h.off_at = (int)up16(sizeof(h) + sizeof(unsigned) * nh);
             h.w_at = (int)up16(h.off_at + sizeof(uint16_t) * off.size());
-            const size_t bytes = up16(h.w_at + sizeof(R) * w.size()), at = p.blob.size();
-            p.blob_at.push_back((int)(at / 16));
-            p.blob.resize(at + bytes);
-            unsigned char *b = p.blob.data() + at;
+            const size_t bytes = up16(h.w_at + sizeof(R) * w.size()), to = p.blob.size();
+            p.blob_at.push_back((int)(to / 16));
+            p.blob.resize(to + bytes);
+            unsigned char *b = p.blob.data() + to;
             std::memcpy(b, &h, sizeof(h));
             std::memcpy(b + sizeof(h), end.data(), sizeof(unsigned) * (h1 - h0));
             if (!off.empty()) {
@@ -106,68 +139,101 @@ inline bool delay_blobs(DelayPlan &p, int n, const double *sc, const std::vector
     return true;
 }
 
-// Chooses the tile and launch shape and builds the lists.  sc [n_scs][n*n] (row =
-// source), delay [n_tables][n*n] steps (>= 1).  As many CTAs per SM as the batch can
+// Whether a pair's simulations are for the kernel, by its longest near list and most sources
+// of a target: in FP32 up to a quarter near (and 8 in any case), in FP64 up to 0.56.  The
+// step loop takes an entry of the near list at a time from L1 or L2, 400 and more cycles
+// where a barrier is due every step, and the per-step kernel all sources at once.  ms per
+// simulated second, 148 simulations, delay / per-step kernel (velocity in m/s: near of all):
+// FP32 200 nodes, 30 %: 12 (10 of 89) 23.5 / 55, 15 (14 of 93) 29 / 51, 20 (31 of 102) 71 / 46,
+// 40 (69 of 102) 141 / 39; FP32 1,000 nodes, 10 %: 15 (33 of 156) 151 / 247; FP64 200 nodes: 20
+// 47 / 95, 30 (58 of 113) 75 / 92, 40 86 / 90; FP64 400 nodes, 20 %: 40 (99 of 137) 139 / 128.
+template <class R>
+inline bool delay_pair_fits(int near, int all) {
+    return near <= std::max(8.0, (sizeof(R) == 4 ? 0.25 : 0.56) * all);
+}
+
+// Chooses the simulations that run on the kernel, the tile and launch shape, and builds the
+// lists.  sc [n_scs][n*n] (row = source), delay [n_tables][n*n] steps (>= 1).  A pair (SC,
+// delay table) is taken if delay_pair_fits and its windows leave tiles of at least 4 sources,
+// whatever else is in the batch.  As many CTAs per SM as the batch can
 // fill while a tile still holds about three entries per target (each target and tile costs
 // a read and a write of its sums and half an entry of padding); alone on its SM a CTA
-// keeps two tile buffers.  Returns false where the kernel does
-// not apply: tiles of under 4 sources, most pairs near, or lists beyond max_bytes.
+// keeps two tile buffers.  Returns false where no simulation is taken, the lists exceed
+// max_bytes (counted before they are built), or of a batch larger than the GPU's SMs most
+// are not taken: the two kernels then run one after the other, and what is left of the
+// per-step kernel's batch takes about as long as all of it (FP32, 500 simulations of 68 nodes
+// at 10-60 m/s: 45 ms per simulated second in two, 33 on the per-step kernel).
 template <class R>
 inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int sms, const double *sc, const int *sc_of,
-                             const std::vector<int> &delay, const std::vector<int> &table_of, int max_delay,
-                             size_t max_bytes) {
-    p.window = (std::max(max_delay, DELAY_BLOCK) + DELAY_BLOCK - 1) / DELAY_BLOCK * DELAY_BLOCK;
-    const auto pairs = delay_pairs(p, n_sims, sc_of, table_of);
+                             const std::vector<int> &delay, const std::vector<int> &table_of, size_t max_bytes) {
+    std::vector<std::pair<int, int>> pairs = delay_pairs(p, n_sims, sc_of, table_of);
     const size_t nn = (size_t)n * n;
+    const int rows = (int)(sizeof(R) * n * (DELAY_BLOCK + 1) + 15) & ~15;
+    // sums of half the targets where two passes over them are possible
+    const double least_rows = sizeof(R) == 4 && n > 512 ? rows / 2 : rows;
     // near lists (d < DELAY_BLOCK) for the steps within a block, by rank q: counted first
-    p.near_cnt.assign(p.n_pairs, 0);
-    p.near_min.assign(p.n_pairs, DELAY_BLOCK);
-    size_t nnz = 0;   // of the fullest pair
-    if ((size_t)p.n_pairs * nn > max_bytes) return false;
-    std::vector<int> near(n), all(n);
-    for (int q = 0; q < p.n_pairs; ++q) {
-        const double *S = sc + (size_t)pairs[q].first * nn;
+    std::vector<int> new_id(pairs.size(), -1);
+    std::vector<std::pair<int, int>> taken;
+    DelayColumns cols;
+    size_t nnz = 0, entries = 0;   // of the fullest pair, of all
+    int max_delay = 1;
+    for (size_t q = 0; q < pairs.size(); ++q) {
+        cols.load(sc, pairs[q].first, n);
         const int *d = delay.data() + (size_t)pairs[q].second * nn;
-        std::fill(near.begin(), near.end(), 0);
-        std::fill(all.begin(), all.end(), 0);
-        for (int k = 0; k < n; ++k)
-            for (int j = 0; j < n; ++j) {
-                if (S[(size_t)k * n + j] == 0.0) continue;
-                const int dk = d[(size_t)k * n + j];
-                ++all[j];
-                if (dk >= DELAY_BLOCK) continue;
-                ++near[j];
-                p.near_min[q] = std::min(p.near_min[q], dk);
+        int least = DELAY_BLOCK, most = 1, cnt = 0;
+        for (int j = 0; j < n && delay_pair_fits<R>(cnt, cols.full); ++j) {
+            int near = 0;
+            for (int e = cols.at[j]; e < cols.at[j + 1]; ++e) {
+                const int dk = d[(size_t)cols.src[e] * n + j];
+                most = std::max(most, dk);
+                near += dk < DELAY_BLOCK;
+                least = std::min(least, dk);
             }
-        p.near_cnt[q] = *std::max_element(near.begin(), near.end());
-        p.far_max = std::max(p.far_max, *std::max_element(all.begin(), all.end()) - p.near_cnt[q]);
-        size_t sum = 0;
-        for (int c : all) sum += c;
-        nnz = std::max(nnz, sum);
+            cnt = std::max(cnt, near);
+        }
+        const int stride = delay_stride((most + DELAY_BLOCK - 1) / DELAY_BLOCK * DELAY_BLOCK), few = std::min(n, 4);
+        const double bytes = least_rows + n * (4 + 0.6 * (2 + sizeof(R))) + 2048 +
+                             few * (stride * (double)sizeof(R) + 1.2 * cols.full * (2 + sizeof(R)));
+        if (!delay_pair_fits<R>(cnt, cols.full) || bytes > DELAY_SMEM_SM || few * (long long)stride > 65535) continue;
+        new_id[q] = (int)taken.size();
+        taken.push_back(pairs[q]);
+        p.near_cnt.push_back(cnt);
+        p.near_min.push_back(least);
+        p.near_k = std::max(p.near_k, cnt);
+        max_delay = std::max(max_delay, most);
+        nnz = std::max(nnz, cols.src.size());
+        entries += cols.src.size();
     }
-    for (int c : p.near_cnt) p.near_k = std::max(p.near_k, c);
-    if (p.near_k > std::max(8, p.far_max / 4) || (size_t)p.n_pairs * p.near_k * n * 16 > max_bytes) return false;
+    for (int s = 0; s < n_sims; ++s) {
+        p.pair[s] = new_id[p.pair[s]];
+        (p.pair[s] >= 0 ? p.sims : p.rest).push_back(s);
+    }
+    p.n_pairs = (int)taken.size();
+    pairs = taken;
+    if (p.sims.empty() || entries * (2 + sizeof(R)) > max_bytes || (size_t)p.n_pairs * p.near_k * n * 16 > max_bytes) return false;
+    if (n_sims > sms && 2 * p.rest.size() > (size_t)n_sims) return false;
+    n_sims = (int)p.sims.size();
+    p.window = (max_delay + DELAY_BLOCK - 1) / DELAY_BLOCK * DELAY_BLOCK;
     p.near.assign((size_t)p.n_pairs * p.near_k * n, 0);
     p.near_w.assign(p.near.size(), 0.0);
     for (int q = 0; q < p.n_pairs; ++q) {
-        const double *S = sc + (size_t)pairs[q].first * nn;
-        const int *d = delay.data() + (size_t)pairs[q].second * nn;
         if (p.near_cnt[q] == 0) continue;
-        std::fill(near.begin(), near.end(), 0);
-        for (int k = 0; k < n; ++k)
-            for (int j = 0; j < n; ++j) {
-                const double v = S[(size_t)k * n + j];
-                const int dk = d[(size_t)k * n + j];
-                if (v == 0.0 || dk >= DELAY_BLOCK) continue;
-                const size_t at = ((size_t)q * p.near_k + near[j]++) * n + j;
-                p.near[at] = k * DELAY_BLOCK + dk;
-                p.near_w[at] = v;
+        cols.load(sc, pairs[q].first, n);
+        const int *d = delay.data() + (size_t)pairs[q].second * nn;
+        for (int j = 0; j < n; ++j) {
+            int rank = 0;
+            for (int e = cols.at[j]; e < cols.at[j + 1]; ++e) {
+                const int k = cols.src[e], dk = d[(size_t)k * n + j];
+                if (dk >= DELAY_BLOCK) continue;
+                const size_t to = ((size_t)q * p.near_k + rank++) * n + j;
+                p.near[to] = k * DELAY_BLOCK + dk;
+                p.near_w[to] = cols.w[e];
             }
+        }
     }
     // tile and launch shape
     const int least = (n + 31) / 32 * 32, stride = delay_stride(p.window);
     const bool f64 = sizeof(R) == 8;
-    const int rows = (int)(sizeof(R) * n * (DELAY_BLOCK + 1) + 15) & ~15;
     const double nnz_node = (double)nnz / n;
     const int thr_sm = f64 ? 512 : 1024;   // by registers, see min_ctas
     const int step_bytes = (int)sizeof(R) * n * n_noise;   // noise of a step
@@ -196,7 +262,7 @@ inline bool build_delay_plan(DelayPlan &p, int n, int n_sims, int n_noise, int s
         const int most = c == 1 ? (f64 ? 512 : n <= 256 ? 512 : 1024) : std::min(f64 ? 256 : 512, thr_sm / c / 32 * 32);
         p.threads = std::max(least, most);
         for (int shrink = 0; shrink < 8 && p.tile_src >= 1; ++shrink) {
-            if (!delay_blobs<R>(p, n, sc, delay, pairs, max_bytes)) return false;
+            if (!delay_blobs<R>(p, n, sc, delay, pairs, cols, max_bytes)) return false;
             p.buf_bytes = ((p.blob_max + p.tile_src * stride * (int)sizeof(R)) + 15) & ~15;
             p.smem = p.buf_at + p.bufs * p.buf_bytes;
             if (p.smem <= most_smem) {

@@ -118,7 +118,9 @@ struct IntegrateArgs {
     BWConst bw;
     ModelK K;
     ModelKf Kf;                  // K rounded to float
-    int sim_begin;               // first simulation of this launch (FP64 kernel)
+    int sim_begin;               // first simulation of this launch (per-simulation kernel)
+    const int *sim_list;         // or the simulations of this launch (per-simulation and delay kernels)
+    int sim_list_n;
     int n_regional;              // regional parameters of the model
     const int *tiles;            // tile kernels: [n_tiles][1 + width] = SC index, then simulation ids (-1 = empty)
     int n_tiles;

@@ -234,11 +234,12 @@ __global__ void __launch_bounds__(MAXT, min_ctas<R, MAXT>()) k_integrate_delay(c
     const size_t ext = a.states_ts ? (size_t)n * a.states_len : (size_t)n;
     const int total = a.bw_it * a.inner_it;
 
-    for (int sim = blockIdx.x; sim < a.n_sims; sim += gridDim.x) {
+    for (int i = blockIdx.x; i < a.sim_list_n; i += gridDim.x) {
+        const int sim = a.sim_list[i];
         const int pair = a.db_pair[sim];                       // (SC, delay table) of this simulation
         const int *const near_off = a.db_near + (size_t)pair * a.db_near_k * n;   // k * 32 + d, padding 0 (d = 0)
         const R *const near_w = A::near_w(a) + (size_t)pair * a.db_near_k * n;
-        const int near_n = a.db_near_cnt ? a.db_near_cnt[pair] : 0;               // longest near list
+        const int near_n = a.db_near_cnt[pair];               // longest near list
         const int sync_every = near_n ? a.db_near_min[pair] : DB;
         int no[NEAR_REGS];   // this node's first near pairs
         R nw[NEAR_REGS];
@@ -464,7 +465,7 @@ cudaError_t config_model(const IntegrateArgs &a, int sms, DelayLaunch *c) {
                                               : occupancy<M, R, 1024>(*c, &occ);
     if (e != cudaSuccess) return e;
     if (occ < 1) return cudaErrorInvalidConfiguration;
-    c->grid = std::min(a.n_sims, occ * sms);
+    c->grid = std::min(a.sim_list_n, occ * sms);
     return cudaSuccess;
 }
 

@@ -104,9 +104,11 @@ __device__ __forceinline__ float coupling_tree16(const float *__restrict__ SC, c
 // so that the BOLD is theirs bit for bit.  Elsewhere their registers cost more than they
 // give: WC 300 nodes, 200 sims, 148 ms per simulated second against 85; rWW 390 nodes,
 // 25 %, 123 against 84.
-template <class M, bool DELAY, class R, bool SPARSE, int MAXT, bool ADJ = false>
+// LIST = the simulations of a.sim_list (delays, beside the delay kernel) instead of
+// consecutive ones, whose index needs no register.
+template <class M, bool DELAY, class R, bool SPARSE, int MAXT, bool ADJ = false, bool LIST = false>
 __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
-    const int sim = a.sim_begin + blockIdx.x;
+    const int sim = LIST ? a.sim_list[blockIdx.x] : a.sim_begin + blockIdx.x;
     const int j = threadIdx.x;
     const int n = a.nodes;
     const bool act = j < n;
@@ -327,6 +329,13 @@ __global__ void __launch_bounds__(MAXT) k_integrate_sim(const IntegrateArgs a) {
 
 template <class M, class R, int MAXT, bool DELAY>
 cudaError_t launch_sim_variant(const IntegrateArgs &a, int grid, int threads, size_t smem, cudaStream_t st) {
+    if constexpr (DELAY && !M::OSC) {
+        if (a.sim_list) {
+            if (a.ell_k > 0) k_integrate_sim<M, true, R, true, MAXT, false, true><<<grid, threads, smem, st>>>(a);
+            else k_integrate_sim<M, true, R, false, MAXT, false, true><<<grid, threads, smem, st>>>(a);
+            return cudaGetLastError();
+        }
+    }
     if (a.ell_k > 0) k_integrate_sim<M, DELAY, R, true, MAXT><<<grid, threads, smem, st>>>(a);
     else k_integrate_sim<M, DELAY, R, false, MAXT><<<grid, threads, smem, st>>>(a);
     return cudaGetLastError();
@@ -343,7 +352,7 @@ template <class M, class R, bool UNCAP>
 cudaError_t launch_sim_kernel(const IntegrateArgs &a, cudaStream_t st) {
     const int threads = ((a.nodes + 31) / 32) * 32;
     const size_t smem = a.has_delay ? 0 : sizeof(typename M::S) * a.nodes;
-    const int grid = a.n_sims - a.sim_begin;
+    const int grid = a.sim_list ? a.sim_list_n : a.n_sims - a.sim_begin;
     if constexpr (std::is_same<M, RWWm<float>>::value) {
         if (!a.has_delay && a.ell_k == 0 && !a.do_fic && a.nodes <= ADJ_REG_NODES) {
             k_integrate_sim<M, false, R, false, 1024, true><<<grid, threads, smem, st>>>(a);

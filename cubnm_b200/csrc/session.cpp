@@ -341,6 +341,8 @@ struct Session {
     bool ready = false;
     int dev = -1;                // the device the stream, events and buffers belong to
     cudaStream_t st = nullptr;
+    cudaStream_t st_rest = nullptr;   // simulations beside the delay kernel's, joined to st by ev_rest
+    cudaEvent_t ev_rest = nullptr;
     cudaEvent_t ev[8];
     // noise cache (bnm.cu:1207-1215 key)
     bool noise_valid = false, noise_f32_valid = false;
@@ -356,7 +358,7 @@ struct Session {
     DBuf d_bold, d_states, d_gbools, d_gints, d_fc, d_fcd, d_wfc, d_pairs_i, d_pairs_j, d_wstart, d_wend, d_status;
     DBuf d_tiles, d_sct_f32, d_ell_pk, d_bw_scr, d_ln_groups, d_ln_params, d_ln_hist, d_ln_bw;
     DBuf fl_ec, fl_q, fl_win, fl_scr;  // fit loss
-    DBuf d_db_pair, d_db_at, d_db_blob, d_db_sums, d_db_near, d_db_near_w, d_db_near_n;  // delay kernel lists
+    DBuf d_db_sims, d_db_hist, d_db_pair, d_db_at, d_db_blob, d_db_sums, d_db_near, d_db_near_w, d_db_near_n;  // delay kernel lists
     DBuf d_pidx, d_wstat;              // tensor-core FC: pair index of (i, j); window-FC statistics
     // gof
     DBuf g_simfc, g_empfc, g_simfcd, g_empfcd, g_out;
@@ -429,10 +431,14 @@ static void close_session(Session *&p) {
                         &S.d_hist, &S.d_hist_f32, &S.d_bold, &S.d_states, &S.d_gbools, &S.d_gints, &S.d_fc,
                         &S.d_fcd, &S.d_wfc, &S.d_pairs_i, &S.d_pairs_j, &S.d_wstart, &S.d_wend, &S.d_status, &S.d_tiles,
                         &S.d_sct_f32, &S.d_ell_pk, &S.d_bw_scr, &S.d_ln_groups, &S.d_ln_params, &S.d_ln_hist, &S.d_ln_bw, &S.fl_ec, &S.fl_q, &S.fl_win, &S.fl_scr, &S.d_pidx, &S.d_wstat,
-                        &S.d_bw_tab, &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_sums, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
+                        &S.d_bw_tab, &S.d_db_sims, &S.d_db_hist, &S.d_db_pair, &S.d_db_at, &S.d_db_blob, &S.d_db_sums, &S.d_db_near, &S.d_db_near_w, &S.d_db_near_n,
                         &S.g_simfc, &S.g_empfc, &S.g_simfcd, &S.g_empfcd, &S.g_out})
             b->release();
         for (auto &ev : S.ev) cudaEventDestroy(ev);
+        if (S.st_rest) {
+            cudaStreamDestroy(S.st_rest);
+            cudaEventDestroy(S.ev_rest);
+        }
         cudaStreamDestroy(S.st);
         if (cur >= 0 && cur != S.dev) cudaSetDevice(cur);
     }
@@ -1078,22 +1084,43 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         round_decline(*t_round);
     }
     // Delayed networks run in blocks of 32 steps (integrate_delay.cuh) unless a kernel
-    // or coupling form is forced; the phase model, whose coupling depends on the
-    // target's current phase, keeps the per-step loop, as do networks of which most
-    // delays are below a block, and FP64 networks whose rows do not fit shared memory.
+    // or coupling form is forced.  The phase model, whose coupling depends on the target's
+    // current phase, keeps the per-step loop, as do the simulations whose delays the plan
+    // does not take (`rest`: too many of a target's are below a block, or the windows of
+    // four sources do not fit shared memory), beside the others, and FP64 networks whose
+    // rows do not fit shared memory.
     DelayPlan plan;
     bool delay_blocks = has_delay && !md.osc && !use_lanes && !force_simt && !coupling_forced;
     if (delay_blocks) {
-        const int *sc_of = host_sc_idx();
-        const double *sc_host = host_sc();
-        const int dmax = *std::max_element(h_max_delay.begin(), h_max_delay.end());
         const size_t most = (size_t)1 << 30;
-        delay_blocks = c.fp32 ? build_delay_plan<float>(plan, n, N, md.n_noise, sm_count(), sc_host, sc_of, h_delay,
-                                                        h_delay_idx, dmax, most)
-                              : build_delay_plan<double>(plan, n, N, md.n_noise, sm_count(), sc_host, sc_of, h_delay,
-                                                         h_delay_idx, dmax, most);
+        delay_blocks = (c.fp32 ? build_delay_plan<float> : build_delay_plan<double>)(
+            plan, n, N, md.n_noise, sm_count(), host_sc(), host_sc_idx(), h_delay, h_delay_idx, most);
+        if (!delay_blocks) plan.rest.clear();
     }
-    if (has_delay && !delay_blocks) {
+    const std::vector<int> &rest = plan.rest;
+    const bool per_step = !delay_blocks || !rest.empty();   // some simulations run on the per-step kernel
+    if (delay_blocks && per_step) {   // its tables and ring buffers: those of the rest alone
+        std::vector<int> id(h_delay.size() / nn, -1), kept;
+        hist_total = 0;
+        std::vector<char> in_rest(N, 0);
+        for (int s : rest) in_rest[s] = 1;
+        for (int s = 0; s < N; ++s) {
+            if (!in_rest[s]) {
+                h_max_delay[s] = h_delay_idx[s] = 0;
+                continue;
+            }
+            int &t = id[h_delay_idx[s]];
+            if (t < 0) {
+                t = (int)(kept.size() / nn);
+                kept.insert(kept.end(), h_delay.begin() + h_delay_idx[s] * nn, h_delay.begin() + (h_delay_idx[s] + 1) * nn);
+            }
+            h_delay_idx[s] = t;
+            h_hist_off[s] = hist_total;
+            hist_total += (long long)h_max_delay[s] * n;
+        }
+        h_delay.swap(kept);
+    }
+    if (has_delay && per_step) {
         S.d_delay.ensure(sizeof(int) * h_delay.size());
         CK(cudaMemcpyAsync(S.d_delay.p, h_delay.data(), sizeof(int) * h_delay.size(), cudaMemcpyHostToDevice, S.st));
         S.d_delay_idx.ensure(sizeof(int) * N);
@@ -1176,11 +1203,19 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         ia.sc_f32 = S.d_sc_f32.as<float>();
     }
     DelayLaunch dl{};
+    IntegrateArgs ia_rest = ia;   // of the per-step launch beside the delay kernel's
     if (delay_blocks) {
         auto up = [&](DBuf &b, const void *p, size_t bytes) {
             b.ensure(bytes);
             CK(cudaMemcpyAsync(b.p, p, bytes, cudaMemcpyHostToDevice, S.st));
         };
+        std::vector<int> lists(plan.sims);
+        lists.insert(lists.end(), rest.begin(), rest.end());
+        up(S.d_db_sims, lists.data(), sizeof(int) * lists.size());
+        ia.sim_list = S.d_db_sims.as<int>();
+        ia.sim_list_n = (int)plan.sims.size();
+        ia_rest.sim_list = ia.sim_list + ia.sim_list_n;
+        ia_rest.sim_list_n = (int)rest.size();
         up(S.d_db_pair, plan.pair.data(), sizeof(int) * plan.pair.size());
         up(S.d_db_at, plan.blob_at.data(), sizeof(int) * plan.blob_at.size());
         up(S.d_db_blob, plan.blob.data(), plan.blob.size());
@@ -1205,10 +1240,10 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
             ia.db_sums = S.d_db_sums.ensure((c.fp32 ? sizeof(float) : sizeof(double)) * (size_t)dl.grid * DELAY_BLOCK * ((n + 3) & ~3));
         if (c.fp32) {
             ia.db_near_w32 = S.d_db_near_w.as<float>();
-            ia.hist_f32 = (float *)S.d_hist_f32.ensure(sizeof(float) * slots);
+            ia.hist_f32 = (float *)S.d_db_hist.ensure(sizeof(float) * slots);
         } else {
             ia.db_near_w64 = S.d_db_near_w.as<double>();
-            ia.hist = (double *)S.d_hist.ensure(sizeof(double) * slots);
+            ia.hist = (double *)S.d_db_hist.ensure(sizeof(double) * slots);
         }
         CK(cudaStreamSynchronize(S.st));  // host vectors go out of scope
     }
@@ -1216,7 +1251,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     // (integrate_tile64.cu) unless a coupling form of the per-simulation kernel is forced.
     const bool t64 = !c.fp32 && !has_delay && !num_fic && tile64_supported(md.id, n) && !coupling_forced;
     bool t64_tiles = false;
-    if (!use_tc && !delay_blocks && !t64) {
+    if (!use_tc && per_step && !t64) {
+        IntegrateArgs &ia_step = delay_blocks ? ia_rest : ia;
         // Sparse coupling for the per-simulation kernels (ELLPACK by target node):
         // used when the densest column of every SC holds at most half the nodes
         // (CBNM_COUPLING=sparse|dense overrides).  Zero weights are skipped and the
@@ -1271,10 +1307,10 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
             S.d_ell_pk.ensure(bytes);
             CK(cudaMemcpyAsync(S.d_ell_pk.p, c.fp32 ? (const void *)pk32.data() : (const void *)pk64.data(), bytes,
                                cudaMemcpyHostToDevice, S.st));
-            if (c.fp32) ia.ell_pk32 = S.d_ell_pk.as<int2>();
-            else ia.ell_pk64 = S.d_ell_pk.as<int4>();
-            ia.ell_k = K;
-            ia.ell_tables = tabs;
+            if (c.fp32) ia_step.ell_pk32 = S.d_ell_pk.as<int2>();
+            else ia_step.ell_pk64 = S.d_ell_pk.as<int4>();
+            ia_step.ell_k = K;
+            ia_step.ell_tables = tabs;
             CK(cudaStreamSynchronize(S.st));  // host vectors go out of scope
         }
     }
@@ -1388,6 +1424,24 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     } else if (delay_blocks) {
         CK(cudaEventRecord(S.ev[1], S.st));
         CK((c.fp32 ? launch_delay32 : launch_delay64)(md.id, ia, dl, S.st));
+        if (!rest.empty()) {
+            // beside the delay kernel's where each simulation has an SM to itself, else after
+            // them: its shared memory would leave the per-step kernel no L1 (FP32, 592
+            // simulations of 100 nodes at 4-40 m/s: 104 ms per simulated second at once)
+            const bool beside = N <= sm_count();
+            if (beside && !S.st_rest) {
+                CK(cudaStreamCreateWithFlags(&S.st_rest, cudaStreamNonBlocking));
+                CK(cudaEventCreateWithFlags(&S.ev_rest, cudaEventDisableTiming));
+            }
+            const cudaStream_t st = beside ? S.st_rest : S.st;
+            if (beside) CK(cudaStreamWaitEvent(st, S.ev[1], 0));
+            CK((c.fp32 ? launch_integrate_simt32 : launch_integrate_fp64)(md.id, ia_rest, st));
+            if (beside) {
+                CK(cudaEventRecord(S.ev_rest, st));
+                CK(cudaStreamWaitEvent(S.st, S.ev_rest, 0));
+            }
+            ++launches;
+        }
         ++launches;
     } else if (c.fp32) {
         CK(cudaStreamSynchronize(S.st));
@@ -1409,7 +1463,8 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
     t_last_kernel = use_pp ? (pp_ws ? "k_integrate_pp_ws" : "k_integrate_pp")
                     : use_tc ? (tc_wide ? "k_integrate_tc" : "k_integrate_mma")
                     : use_lanes ? "k_integrate_lanes"
-                    : delay_blocks ? (plan.passes == 2 ? "k_integrate_delay/2" : "k_integrate_delay")
+                    : delay_blocks ? std::string(plan.passes == 2 ? "k_integrate_delay/2" : "k_integrate_delay") +
+                                         (rest.empty() ? "" : "+k_integrate_sim")
                     : t64 ? (t64_tiles ? "k_tile64" : "k_one64") : "k_integrate_sim";
     CK(cudaEventRecord(S.ev[2], S.st));
     if (!device_io) {  // the integrator runs asynchronously: map the host output pages meanwhile

@@ -1,6 +1,6 @@
 // Walks the delay kernel's lists (delay_plan.h) as its gather does and compares every sum
 // with the direct one: prints one line per plan, "plan accepted passes tile_src tiles
-// threads smem near_k" and "sum <hash of all sums>", and returns 1 on any difference.
+// threads smem near_k rest" and "sum <hash of all sums>", and returns 1 on any difference.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -17,28 +17,33 @@ static int check(int n, int n_sims, int sms, double density, int dmin, int dmax,
     std::vector<double> sc(nn);
     for (double &v : sc) v = u(g) < density ? u(g) : 0.0;
     std::vector<int> delay(nn * tables), sc_of(n_sims, 0), table_of(n_sims);
-    int most = 0;
-    for (int t = 0; t < tables; ++t)
+    for (int t = 0; t < tables; ++t)   // table t: the first one's delays at (t + 1) times the speed
         for (size_t i = 0; i < nn; ++i) {
-            delay[t * nn + i] = dmin + (int)(u(g) * (dmax - dmin + 1));
-            most = std::max(most, delay[t * nn + i]);
+            delay[t * nn + i] = t ? std::max(1, delay[i] / (t + 1)) : dmin + (int)(u(g) * (dmax - dmin + 1));
         }
     for (int s = 0; s < n_sims; ++s) table_of[s] = s % tables;
     DelayPlan p;
-    const bool ok = build_delay_plan<R>(p, n, n_sims, n_noise, sms, sc.data(), sc_of.data(), delay, table_of, most, (size_t)1 << 30);
-    std::printf("plan %d passes %d tile_src %d tiles %d threads %d smem %d near_k %d", ok, p.passes, p.tile_src, p.tiles, p.threads,
-                p.smem, p.near_k);
+    const bool ok = build_delay_plan<R>(p, n, n_sims, n_noise, sms, sc.data(), sc_of.data(), delay, table_of, (size_t)1 << 30);
+    std::printf("plan %d passes %d tile_src %d tiles %d threads %d smem %d near_k %d rest %d", ok, p.passes, p.tile_src, p.tiles, p.threads,
+                p.smem, p.near_k, (int)p.rest.size());
     if (!ok) {
         std::printf(" sum 0\n");
         return 0;
     }
+    std::vector<int> table(p.n_pairs, -1);   // delay table of each pair that is taken
+    int most = 0;
+    for (int s : p.sims) table[p.pair[s]] = table_of[s];
+    for (int t : table)
+        for (size_t i = 0; i < nn; ++i)
+            if (sc[i] != 0.0) most = std::max(most, delay[t * nn + i]);
+    if ((int)(p.sims.size() + p.rest.size()) != n_sims) return 1;
     const int W = p.window, WS = delay_stride(W), nh = (n + p.passes - 1) / p.passes;
     if (p.smem > DELAY_SMEM_SM - 1024 || p.tile_src * WS > 65536 || W < most) return 1;
     std::vector<R> x((size_t)n * (W + DELAY_BLOCK));   // x_k(t0 - W + i); i >= W: this block's values
     for (R &v : x) v = (R)u(g);
     uint64_t hash = 1469598103934665603ull;
     for (int q = 0; q < p.n_pairs; ++q) {
-        const int *d = delay.data() + (size_t)q * nn;
+        const int *d = delay.data() + (size_t)table[q] * nn;
         for (int pass = 0; pass < p.passes; ++pass) {
             const int h0 = pass * nh, h1 = std::min(n, h0 + nh);
             std::vector<R> row((size_t)(h1 - h0) * 32, R(0));

@@ -36,8 +36,21 @@ def test_lists_give_the_direct_sums_in_any_batch(check, precision, nodes, densit
     assert len({p["sum"] for p in plans}) == 1, plans
 
 
-def test_several_delay_tables(check):
-    assert check("double", 60, 50, 148, 0.4, 10, 200, 7, 2)["plan"] == "1"
+@pytest.mark.parametrize("precision", ["float", "double"])
+def test_only_near_heavy_tables_are_left_out(check, precision):
+    """Delays of 60-400 steps and 2 to 20 times as fast, five simulations of each: the fast
+    tables' simulations are left to the per-step kernel, the others stay."""
+    p = check(precision, 60, 100, 148, 0.4, 60, 400, 20, 2)
+    assert p["plan"] == "1" and 0 < int(p["rest"]) < 100
+    assert check(precision, 60, 400, 148, 0.4, 60, 400, 20, 2)["plan"] == "0"   # most of a large batch
+    q = check(precision, 60, 5, 148, 0.4, 60, 400, 1, 2)   # the slowest alone
+    assert q["rest"] == "0"
+
+
+def test_one_slow_table_does_not_decide_for_the_others(check):
+    """Delays to 12,000 steps leave no tile of four sources, half of them do."""
+    p = check("double", 30, 10, 148, 0.5, 100, 12000, 2, 2)
+    assert (p["plan"], p["rest"]) == ("1", "5")
 
 
 def test_two_passes_are_planned(check):

@@ -79,3 +79,31 @@ def test_two_passes_over_the_targets(nodes, density, ms):
     assert core.last_kernel() == "k_integrate_delay/2"
     np.testing.assert_allclose(o32["_sim_states"], o64["_sim_states"], rtol=1e-4, atol=1e-5)
     assert np.abs(o32["sim_bold"] - o64["sim_bold"]).max() < 1e-4
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("fic", [0, 2])
+def test_mixed_velocities_run_on_two_kernels_at_once(precision, fic):
+    """Simulations whose delays are mostly below a block of 32 steps run on the per-step
+    kernel, beside the others: each gives what it gives alone."""
+    nodes, N = 60, 40
+    a = _args("rWW", nodes, N, _uniform(nodes, 60, 300), np.linspace(4.0, 60.0, N), 300, 0.5, precision)
+    a[7] = dict(a[7], do_fic=str(int(fic > 0)), max_fic_trials="3" if fic == 2 else "0", fic_i_sampling_start="50",
+                fic_i_sampling_end="100")
+    b = _copy(a)
+    whole = core.run_simulations(*b)
+    assert core.last_kernel() == "k_integrate_delay+k_integrate_sim"
+    kernels = set()
+    for i in (0, 5, 20, 39):
+        c = _subset(a, np.array([i]))
+        alone = core.run_simulations(*c)
+        kernels.add(core.last_kernel())
+        np.testing.assert_array_equal(alone["sim_bold"], whole["sim_bold"][[i]])
+        np.testing.assert_array_equal(alone["_sim_states"], whole["_sim_states"][:, [i]])
+        np.testing.assert_array_equal(alone["_global_ints"], whole["_global_ints"][:, [i]])
+        np.testing.assert_array_equal(c[5], b[5].reshape(-1, N, nodes)[:, i])   # wIE as written back
+    assert kernels == {"k_integrate_delay", "k_integrate_sim"}
+    if precision == "fp64":
+        pick = np.array([0, 39])
+        ref = oracle.run_simulations(*_subset(a, pick))
+        np.testing.assert_allclose(whole["sim_bold"][pick], ref["sim_bold"], rtol=1e-8, atol=1e-12)
