@@ -365,7 +365,7 @@ struct JR32 {  // jr.cpp:80-133 in FP32
 //                d = nu/c - 1, |d| <= 0.118 (binomial series; error <= 3 ulp)
 //   (1-rho)^(1/f) = (1-rho) exp(t), t = ln(1-rho) (1-f)/f, exp(t) = e^(i/8) exp(t - i/8), the
 //                last by its Taylor series to y^10/10!, |y| <= 1/16 (first omitted term < 1e-18)
-//   1/x        = approximate reciprocal (20 bits) refined by two Newton steps (<= 1 ulp)
+//   1/x        = approximate reciprocal (20 bits) refined by two Newton steps (<= 1.5 ulp)
 // c^-1, c^a and e^(i/8) come from a small table (filled on the host) that covers
 // nu in [0.15, 6.6] and f > 0.17; outside it the general exp2 / log2 forms and IEEE
 // division are used.  Near rest (c = 1, i = 0) the factors are 1.  A series around 1
