@@ -256,7 +256,7 @@ def run_ours(opts, rank, world, local_rank):
                 "sims": n64, "unit": UNIT}
 
     # roofline of the dominant kernel (the integrator).  Its binding resource is the
-    # FP32 / MUFU node update (ncu: profiles/), so the bound reported is FP32 FLOP/s of
+    # FP32 / MUFU node update, so the bound reported is FP32 FLOP/s of
     # the update against this GPU's measured FMA throughput; the coupling GEMM's
     # tensor-pipe fraction is reported beside it.
     peaks = {}
@@ -290,7 +290,7 @@ def run_ours(opts, rank, world, local_rank):
             "traffic": traffic, "traffic_source": traffic_src,
             "algorithmic_bytes": N_SIMS * NODES * DURATION_S * 8.0 if n_sims == N_SIMS else None,
             "kernel": kernel, "kernel_ms": integ * 1e3,
-            "note": "per-pipe utilisation of this kernel: profiles/ (ncu)"}
+            "note": "counters of this kernel: profiles/ (ncu)"}
 
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": opts.steps,
@@ -488,11 +488,27 @@ def _oracle_sample(args, sample, duration_s=None):
     return sample * a[16] / 1000 / el, el
 
 
+def smem_roofline(gather_bytes, seconds):
+    """What bounds the delay kernel's gathers: they are read from shared memory (128 bytes a
+    cycle and SM), where a block's ring buffers are staged, not from HBM."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 148
+    try:
+        mhz = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["sm_max_mhz"]
+    except Exception:
+        mhz = 1965.0
+    peak = sms * 128 * mhz / 1e3
+    return {"achieved": gather_bytes / seconds / 1e9, "peak": peak, "unit": "GB/s",
+            "frac": gather_bytes / seconds / 1e9 / peak,
+            "peak_source": f"nominal: {sms} SMs x 128 B a cycle at {mhz:.0f} MHz"}
+
+
 def config_roofline(args, integrate_ms, delayed, fp32_peak=None):
     """Roofline of the integrator of a c2-c4 workload (per launch, mean CUDA-event
     time of the integrator).  Delayed networks: the ring-buffer gathers, 4 bytes per
-    nonzero of the target's SC column per node-step, against the measured HBM copy
-    bandwidth (no credit taken for L2 hits).  Without delays (c3): the FP32 work of a
+    nonzero of the target's SC column per node-step, as if each were an HBM access, against
+    the measured copy bandwidth, and under "smem" against the shared memory that serves
+    them in the delay kernel.  Without delays (c3): the FP32 work of a
     node-step (2 flops per nonzero of the coupling + the rWW update) against the
     measured FP32 peak."""
     from cubnm_b200 import core
@@ -507,7 +523,7 @@ def config_roofline(args, integrate_ms, delayed, fp32_peak=None):
         b = node_steps * nnz * 4.0
         return {"bound": "hbm", "achieved": b / t / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": b / t / 1e9 / peaks["hbm_gbs"], "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
-                "traffic": None, "algorithmic_bytes": b,
+                "traffic": None, "algorithmic_bytes": b, "smem": smem_roofline(b, t),
                 "work": f"{nnz:.1f} ring-buffer gathers x 4 B per node-step (from shared memory, where the "
                         f"delay kernel stages the buffers every 32 steps), {node_steps:.3e} node-steps",
                 "kernel": kernel, "kernel_ms": integrate_ms}
@@ -521,7 +537,8 @@ def config_roofline(args, integrate_ms, delayed, fp32_peak=None):
 def batch_roofline(groups, seconds):
     """Roofline of an uneven batch (c2): the ring-buffer gather bytes of all groups
     (4 bytes per nonzero of the target's SC column per node-step) over the batch's
-    wall time, against the measured HBM bandwidth.  The groups' integrators, FC and
+    wall time, against the measured HBM bandwidth and under "smem" against the shared
+    memory that serves them.  The groups' integrators, FC and
     copies run concurrently on their own streams, so there is no single launch to
     time: this is a lower bound on the gathers' achieved bandwidth."""
     peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -533,7 +550,7 @@ def batch_roofline(groups, seconds):
         b += N * n * (g[16] / g[20]) * nnz * 4.0
     return {"bound": "hbm", "achieved": b / seconds / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": b / seconds / 1e9 / peaks["hbm_gbs"], "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
-            "traffic": None, "algorithmic_bytes": b,
+            "traffic": None, "algorithmic_bytes": b, "smem": smem_roofline(b, seconds),
             "work": "ring-buffer gathers of every group, 4 B per nonzero per node-step (from shared memory, where "
                     "the delay kernel stages the buffers every 32 steps)",
             "basis": "whole-batch wall time (the groups' kernels run concurrently on their own streams)"}
