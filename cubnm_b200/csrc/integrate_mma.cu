@@ -36,8 +36,8 @@
 //
 // mma.sync reaches a quarter of tcgen05's rate on sm_100a (measured 950 FP16 multiply-
 // adds a cycle and SM), but a tile's 147 products at 100 nodes are 316 cycles of it, in
-// the shadow of the other CTA's update.  Measured at 100 nodes: 1,492 cycles a step with
-// one CTA an SM (8 simulations), 2,262 with two (200 nodes, one: 3,930).  What bounds a step then: the phases of a
+// the shadow of the other CTA's update.  Measured at 100 nodes: 1,500 cycles a step with
+// one CTA an SM (8 simulations), 2,290 with two (200 nodes, one: 3,930).  What bounds a step then: the phases of a
 // CTA's warps (product, MUFU, update) follow one another between its barriers, with two
 // CTAs to overlap; more do not fit the registers.
 #include <algorithm>
@@ -150,7 +150,7 @@ __host__ __device__ constexpr bool lo_in_smem(int ks) { return ks > 6; }   // A 
 // registers come from its quarter of the SM), at least one.
 __host__ __device__ constexpr int bw_warps(int mt) { return mt % 4 ? 4 - mt % 4 : mt <= 4 ? 4 : 2; }
 // CTAs an SM should hold: about 128 registers a thread, fewer for 8 node warps.
-__host__ __device__ constexpr int min_ctas(int ks) { return ks <= 4 ? 2 : ks <= 8 ? 2 : 1; }
+__host__ __device__ constexpr int min_ctas(int ks) { return ks <= 8 ? 2 : 1; }
 
 // The Balloon-Windkessel warps: for every tile and millisecond, wait for the inputs of the
 // 8 n items (item s n + j), step them two at a time, write BOLD at TR.

@@ -982,7 +982,7 @@ static void run_impl(Session *sp, const cbnm_run_args *a, cbnm_outputs *o, bool 
         has_delay = *std::max_element(h_max_delay.begin(), h_max_delay.end()) > 0;
     }
     // FP32 kernels: the tensor-core tiles take shared-SC batches without delays or
-    // numerical FIC at <= 224 nodes (200-node rWW, 512 sims: 3,610 cycles a step of the
+    // numerical FIC at <= 224 nodes (200-node rWW, 512 sims: 3,930 cycles a step of the
     // batch against 8,700 on the per-simulation kernel); delayed networks run in blocks of
     // 32 steps (integrate_delay.cuh: 1,000-node WC, 148 sims: 19,700 cycles per sim-step
     // and SM against the lane kernel's 66,000), everything else on the per-simulation

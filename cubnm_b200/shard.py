@@ -4,9 +4,13 @@ Simulations are independent: nothing is exchanged during the time loop, and
 the noise array (segment + shuffles) depends only on the seed, the node count
 and the duration, not on which simulations a process runs.  So a batch is cut
 into contiguous shards of simulations, each rank runs its shard through the
-single-GPU entry point on its own device, and the outputs are gathered.  The
-gathered result equals the one-GPU result of the whole batch, simulation by
-simulation.  The only collectives are the gather of outputs at the end (to one
+single-GPU entry point on its own device, and the outputs are gathered.  In FP64 a
+simulation gives the same bits in any batch, so the gathered result equals the
+one-GPU result of the whole batch, simulation by simulation (delayed batches of which
+most simulations' delays are below 32 steps, and delay lists beyond 1 GiB, change kernel
+as a whole: to rounding then).  In FP32 the kernel also depends on the batch at 113-128
+nodes (more than 16 simulations per SM) and above 128 nodes (simulations per SC), and
+equality there is to rounding.  The only collectives are the gather of outputs at the end (to one
 rank by default) and a MAX of timings; none sits on the data path.
 
 The reference runs a batch on one GPU (src/cubnm/sim/base.py:673-766 calls

@@ -87,12 +87,13 @@ def test_mixed_velocities_run_on_two_kernels_at_once(precision, fic):
     """Simulations whose delays are mostly below a block of 32 steps run on the per-step
     kernel, beside the others: each gives what it gives alone."""
     nodes, N = 60, 40
-    a = _args("rWW", nodes, N, _uniform(nodes, 60, 300), np.linspace(4.0, 60.0, N), 300, 0.5, precision)
-    a[7] = dict(a[7], do_fic=str(int(fic > 0)), max_fic_trials="3" if fic == 2 else "0", fic_i_sampling_start="50",
-                fic_i_sampling_end="100")
+    a = _args("rWW", nodes, N, _uniform(nodes, 60, 300), np.linspace(4.0, 60.0, N), 1200 if fic else 300, 0.5, precision)
+    a[7] = dict(a[7], do_fic=str(int(fic > 0)), max_fic_trials="3" if fic == 2 else "0", I_SAMPLING_START="0",
+                I_SAMPLING_END="1000")
     b = _copy(a)
     whole = core.run_simulations(*b)
     assert core.last_kernel() == "k_integrate_delay+k_integrate_sim"
+    assert not fic or whole["_global_ints"].max() > 0   # trials of the numerical FIC
     kernels = set()
     for i in (0, 5, 20, 39):
         c = _subset(a, np.array([i]))
